@@ -362,10 +362,10 @@ class _Neighbours:
     the padded row ``idx`` of its neighbours' numbers there (-1: none)."""
 
     def __init__(self, s, rc, device):
-        box = torch.as_tensor(s.box, dtype=torch.float64, device=device)
-        f = torch.as_tensor(s.x, dtype=torch.float64, device=device) @ torch.linalg.inv(box)
+        box, inverse = (torch.as_tensor(a, dtype=torch.float64, device=device) for a in (s.box, np.linalg.inv(s.box)))
+        f = torch.as_tensor(s.x, dtype=torch.float64, device=device) @ inverse
         f = f - torch.floor(f)
-        reach = rc * torch.linalg.norm(torch.linalg.inv(box), dim=0)
+        reach = rc * inverse.square().sum(0).sqrt()
         R = [int(math.ceil(float(v))) for v in reach]
         n = len(f)
         pos, owner = [f], [torch.arange(n, device=device)]
