@@ -91,6 +91,9 @@ constexpr float kTcAlphaMax = 1024.f;  // largest |alpha| the tensor-core forwar
 #define NNAP_SPH_SHAPES(X)                                                                    \
     X(6, 18, 9) X(4, 18, 9) X(4, 5, 5) X(2, 4, 4) X(2, 8, 4) X(2, 12, 4) X(3, 5, 4) X(2, 16, 4) \
     X(3, 10, 5) X(6, 9, 9) X(4, 9, 9) X(3, 8, 4) X(4, 10, 5)
+// Spherical shapes compiled for evaluation alone: the model format's defaults (nmax 5, lmax 6)
+// with several and with one species.
+#define NNAP_SPH_EVAL_SHAPES(X) X(6, 12, 6) X(6, 6, 6)
 
 // Radial functions of a sub-basis: the NNAP Chebyshev basis or the NEP basis (radial_f /
 // radial_g in sph_math.cuh).
@@ -108,7 +111,8 @@ cudaError_t upload_sh_constants();
 cudaError_t launch_subrows(const PairBufs& P, int n, float rc, float4* sdx, int* spos, int* scount,
                            cudaStream_t st);
 // basis: kRbNNAP or kRbNEP (the radial functions of the sub-basis).
-// desc_compiled: a shape-specialised instance exists (NNAP_*_SHAPES / NEP_*_SHAPES);
+// desc_compiled: a shape-specialised instance of every kernel, training's included, exists
+// (NNAP_RADIAL_SHAPES, NNAP_SPH_SHAPES / NEP_*_SHAPES);
 // desc_supported: that, or the any-shape kernels of k_desc_gen.cu fit in shared memory.
 bool desc_compiled(int kind, int basis, int lmax, int np, int n1);
 bool desc_supported(int kind, int basis, int lmax, int np, int n1);

@@ -560,251 +560,317 @@ __global__ void __launch_bounds__(32 * kDescMaxWarps, 2) k_sph_bwd(DescArgs a) {
 }
 
 // Backward in the space of the radial functions (used when every column of the fuse
-// matrices has at most kNz nonzero rows and N1 < NP, e.g. the default, full, exfull and
-// fuse weight types).  With Gh[tn][lm][n] = sum_p W[tc][tn][p][n] G[p][lm], formed once per
-// atom from the sparse fuse table,
+// matrices has at most kNz nonzero rows, e.g. the default, none, full, exfull and fuse weight
+// types).  With Gh[tn][lm][n] = sum_p W[tc][tn][p][n] G[p][lm], formed once per atom,
 //   dY_lm = sum_p c_p G[p][lm] = fc sum_n T_n Gh[tn][lm][n],
 //   v_n   = sum_p W[p][n] dc_p = sum_lm Gh[tn][lm][n] Y_lm,
 // so the per-neighbour products run over N1 instead of NP channels, and c, dc are never
-// formed.  Y and dY/dtheta are formed row by row from the lane's Legendre column in
-// shared memory with cos/sin(m phi) recurrences, instead of being stored.  The Gh rows of
-// m != 0 are stored times sqrt2 (the factor of those Y_lm) and the Chebyshev values times
-// fc, so the per-neighbour loop multiplies by neither.
+// formed.  The harmonics are the monic ones of sph_math.cuh (their factors N_lm are in the Gh
+// rows), walked column by column in m with everything in registers; the gradient is taken in
+// Cartesian form: with a_m = sum_l Q_lm dY_lm, b_m = sum_l Q_lm dY_l,-m and a'_m, b'_m the same
+// sums over dQ_lm/dz, and c_m + i s_m = (x + iy)^m,
+//   d/dz = sum_m a'_m c_m + b'_m s_m,   d/dx = sum_m m (a_m c_{m-1} + b_m s_{m-1}),
+//   d/dy = sum_m m (b_m c_{m-1} - a_m s_{m-1}),
+// projected onto the sphere at the end.  Rows l,m and l,-m (and two rows of m = 0) sit side by
+// side as float2 in shared memory, so one paired FMA serves both.
+//
+// Every lane reads N1 (L+1)^2 floats of Gh for each neighbour, and shared memory returns 128
+// bytes per cycle and SM: that path is 86 % busy (the FMA pipe 52 %), against the angle-based
+// walk with stored Legendre columns before, which issued twice the instructions.  1024-structure
+// batch (526k atoms, lmax 6) 2.55 -> 1.98 ms, 1M-atom glass (lmax 4) 3.19 -> 1.76 ms, 32000-atom
+// liquid 174 -> 139 us.  Two neighbours of one species per lane halve the reads but leave 11
+// warps per SM (165 registers): 2.45 ms on the batch.
 template <int L, int NP, int N1>
 struct SphNShape {
     static constexpr int K = (L + 1) * (L + 1);
-    static constexpr int NT = L * (L + 1) / 2 + L + 1;      // Legendre entries
-    static constexpr int N1P = (N1 + 3) & ~3;
-    static constexpr int NPS = (NP + 3) & ~3;
-    static constexpr int SCR = ((K * NP > NT * 32 ? K * NP : NT * 32) + 3) & ~3;  // keeps float4 rows aligned
-    static int warp_floats(int T) { return T * K * N1P + SCR; }
+    static constexpr int NZ = (L + 2) / 2;                 // row pairs of m = 0: (0,1), (2,3), ..
+    static constexpr int NS = NZ + L * (L + 1) / 2;        // and of (l, +-m), m ascending
+    static constexpr int RF = (2 * N1 + 3) & ~3;           // floats of a row pair
+    // floats of one neighbour species, an odd number of 16-byte words: lanes of different
+    // species read different banks
+    static constexpr int GH = (NS * RF / 4) % 2 ? NS * RF : NS * RF + 4;
+    static int warp_floats(int T, int apw, bool diag) { return apw * (T * GH + (diag ? 0 : (NP * K + 3) / 4 * 4)); }
 };
 
-template <int L, int NP, int N1>
-__global__ void __launch_bounds__(32 * kDescMaxWarps, 2) k_sph_bwd_n(DescArgs a) {
+// First row pair of column m >= 1 (row pair of l = m).
+template <int L>
+__host__ __device__ constexpr int pair_start(int m) {
+    int s = (L + 2) / 2;
+    for (int q = 1; q < m; ++q) s += L - q + 1;
+    return s;
+}
+
+// sum_n T_n Gh[n] of a row pair, and v_n += Gh[n] Y: the two contractions of the backward.
+template <int N1>
+__device__ __forceinline__ float2 gh_row(const float* __restrict__ gh, const float2* T2, float2 y2, float2* v2) {
+    float2 dy = make_float2(0.f, 0.f);
+    const float4* gr = reinterpret_cast<const float4*>(gh);
+#pragma unroll
+    for (int q = 0; q < N1 / 2; ++q) {
+        const float4 g = gr[q];
+        const float2 ga = make_float2(g.x, g.y), gb = make_float2(g.z, g.w);
+        dy = __ffma2_rn(T2[2 * q], ga, dy);
+        v2[2 * q] = __ffma2_rn(ga, y2, v2[2 * q]);
+        dy = __ffma2_rn(T2[2 * q + 1], gb, dy);
+        v2[2 * q + 1] = __ffma2_rn(gb, y2, v2[2 * q + 1]);
+    }
+    if (N1 & 1) {
+        const float2 ga = *reinterpret_cast<const float2*>(gh + 2 * (N1 - 1));
+        dy = __ffma2_rn(T2[N1 - 1], ga, dy);
+        v2[N1 - 1] = __ffma2_rn(ga, y2, v2[N1 - 1]);
+    }
+    return dy;
+}
+
+// Columns m .. L of the walk: q is column m, (cm, sm) = (x + iy)^m, (cp, sp) the power before.
+template <int L, int N1, int m>
+__device__ __forceinline__ void bwd_columns(const float* __restrict__ gh, const float2* T2, float2* v2, float x, float y,
+                                            float z, const float* q, float cm, float sm, float cp, float sp, float& gx,
+                                            float& gy, float& gz) {
+    constexpr int RF = (2 * N1 + 3) & ~3;
+    float qn[L + 2];  // column m + 1
+    if constexpr (m < L) monic_column<L, m + 1>(z, qn);
+    float2 ab = make_float2(0.f, 0.f), abz = make_float2(0.f, 0.f);
+    const float2 cs = make_float2(cm, sm);
+#pragma unroll
+    for (int l = m; l <= L; ++l) {
+        const float2 q2 = make_float2(q[l], q[l]);
+        const float2 y2 = l == m ? cs : __fmul2_rn(q2, cs);
+        const float2 dy = gh_row<N1>(gh + (pair_start<L>(m) + l - m) * RF, T2, y2, v2);
+        if (l == m) {
+            ab = dy;
+        } else {
+            const float dq = (float)(l - m) * qn[l];
+            ab = __ffma2_rn(q2, dy, ab);
+            abz = __ffma2_rn(make_float2(dq, dq), dy, abz);
+        }
+    }
+    if (m < L) gz = fmaf(abz.x, cm, fmaf(abz.y, sm, gz));
+    gx = fmaf((float)m, fmaf(ab.x, cp, ab.y * sp), gx);
+    gy = fmaf((float)m, fmaf(ab.y, cp, -(ab.x * sp)), gy);
+    if constexpr (m < L)
+        bwd_columns<L, N1, m + 1>(gh, T2, v2, x, y, z, qn, fmaf(x, cm, -(y * sm)), fmaf(x, sm, y * cm), cm, sm, gx, gy,
+                                  gz);
+}
+
+// LPA lanes serve one atom (32 / LPA atoms per warp).  96 registers (20 warps per SM) with 32
+// lanes, 80 (24 warps) with 16: each was the faster of the two for its shapes.
+constexpr int kBwdWarps = 4;  // most warps per CTA
+template <int L, int NP, int N1, int LPA>
+__global__ void __launch_bounds__(32 * kBwdWarps, LPA == 32 ? 5 : 6) k_sph_bwd_n(DescArgs a) {
     pdl_enter();
     using S = SphNShape<L, NP, N1>;
-    extern __shared__ float smem[];
+    constexpr int APW = 32 / LPA;
+    extern __shared__ __align__(16) float smem[];
     const int T = a.T;
-    const int ntab = T * T * N1 * kNz;
-    int* sNp = reinterpret_cast<int*>(smem);
-    float* sNw = smem + ntab;
+    // per row pair: N_lm of its two rows, and N_lm 2 4pi/(2l+1) (zero where there is no row or
+    // no power-spectrum column)
+    float2* sN = reinterpret_cast<float2*>(smem);
+    float2* sCo = sN + S::NS;
+    const bool diag = a.fwd_alpha != nullptr && T <= kFwdTypes;
+    float* tab = smem + ((4 * S::NS + 3) & ~3);
+    const int ntab = diag ? 0 : T * T * N1 * kNz, nal = diag ? T * kFwdTypes * NP : 0;
+    int* sNp = reinterpret_cast<int*>(tab);
+    float* sNw = tab + ntab;
+    float* sAl = tab;  // alpha[tc][tn][p] of fuse rows with their one nonzero in column p mod N1
     for (int q = threadIdx.x; q < ntab; q += blockDim.x) {
         sNp[q] = a.nz_p[q];
         sNw[q] = a.nz_w[q];
     }
-    // fuse rows with their one nonzero in column p mod N1: alpha[tc][tn][p] in shared memory
-    const bool diag = a.fwd_alpha != nullptr && T <= kFwdTypes;
-    const int nal = diag ? T * kFwdTypes * NP : 0;
-    float* sAl = smem + ((2 * ntab + 3) & ~3);
     for (int q = threadIdx.x; q < nal; q += blockDim.x) sAl[q] = a.fwd_alpha[q];
+    for (int s = threadIdx.x; s < S::NS; s += blockDim.x) {
+        int l0, l1, m = 0;
+        if (s < S::NZ) {
+            l0 = 2 * s;
+            l1 = 2 * s + 1;
+        } else {
+            int t = s - S::NZ;
+            for (m = 1; t >= L - m + 1; ++m) t -= L - m + 1;
+            l0 = l1 = m + t;
+        }
+        const float n0 = c_shN[tri(l0, m)], n1 = l1 <= L ? c_shN[tri(l1 <= L ? l1 : 0, m)] : 0.f;
+        sN[s] = make_float2(n0, n1);
+        sCo[s] = make_float2(l0 < a.nl2 ? n0 * (2.f * kPi4 / (float)(2 * l0 + 1)) : 0.f,
+                             l1 < a.nl2 ? n1 * (2.f * kPi4 / (float)(2 * l1 + 1)) : 0.f);
+    }
     __syncthreads();
-    const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int w = blockIdx.x * (blockDim.x >> 5) + wl;
+    const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane / LPA, sub = lane % LPA;
+    const int w0 = (blockIdx.x * (blockDim.x >> 5) + wl) * APW, w = w0 + grp;
     const int s0 = a.range[a.t0], s1 = a.range[a.t1];
-    if (s0 + w >= s1) return;
-    float* sGh = sAl + ((nal + 3) & ~3) + (size_t)wl * (T * S::K * S::N1P + S::SCR);  // [T][K][N1P]
-    float* scr = sGh + T * S::K * S::N1P;   // G [NP][K], then the Legendre columns [NT][32]
-    const int at = a.perm[s0 + w];
+    if (s0 + w0 >= s1) return;
+    const bool act = s0 + w < s1;
+    float* sGh = tab + ((diag ? nal : 2 * ntab) + 3) / 4 * 4 + (size_t)(wl * APW + grp) * (T * S::GH + (diag ? 0 : (NP * S::K + 3) / 4 * 4));
+    const int at = a.perm[act ? s0 + w : s0 + w0];
     const int tc = a.type[at] - 1;
-    const int M = a.P.M, cnt = min(a.P.count[at], M);
+    const int M = a.P.M, cnt = act ? min(a.P.count[at], M) : 0;
+    int cmax = cnt;
+    if (APW > 1) cmax = __reduce_max_sync(0xffffffffu, cnt);
     const float rc = a.rcut, irc = 1.f / a.rcut;
-    if (diag) {
-        // Gh[tn][lm][n] = sum over p = n mod N1 of alpha[tc][tn][p] G[p][lm], with
-        // G[p][lm] = 2 * 4pi/(2l+1) * dE/dfp[p][l] * A[p][lm] held in registers: lanes over lm
+    if (act) {
+        // G[p][lm] = 2 4pi/(2l+1) dE/dfp[p][l] A[p][lm] (+ the invariant columns' part) times N_lm,
+        // in row pairs; lanes over row pairs
         const float* Ain = a.A + (size_t)w * NP * S::K;
+        const float* Gx = a.Gx ? a.Gx + (size_t)w * NP * S::K : nullptr;
         const float* gf = a.gfp + (size_t)(s0 + w) * a.fp_stride + a.fp_off;
-        const float* al = sAl + (size_t)tc * kFwdTypes * NP;
-        for (int lm = lane; lm < S::K; lm += 32) {
-            int l = 0;
-            while ((l + 1) * (l + 1) <= lm) ++l;
-            const float coef = l < a.nl2 ? 2.f * kPi4 / (float)(2 * l + 1) : 0.f;
-            const int lc = l < a.nl2 ? l : 0;
-            float g[NP];
+        for (int s = sub; s < S::NS; s += LPA) {
+            int l0, l1, k0, k1;
+            if (s < S::NZ) {
+                l0 = 2 * s;
+                l1 = min(2 * s + 1, L);
+                k0 = l0 * l0 + l0;
+                k1 = l1 * l1 + l1;
+            } else {
+                int t = s - S::NZ, m = 1;
+                for (; t >= L - m + 1; ++m) t -= L - m + 1;
+                l0 = l1 = m + t;
+                k0 = l0 * l0 + l0 + m;
+                k1 = l0 * l0 + l0 - m;
+            }
+            const float2 co = sCo[s], nm = sN[s];
+            l0 = l0 < a.nl2 ? l0 : 0;
+            l1 = l1 < a.nl2 ? l1 : 0;
+            float2 g[NP];
 #pragma unroll
             for (int p = 0; p < NP; ++p) {
-                g[p] = coef * gf[p * a.sl + lc] * Ain[p * S::K + lm];
-                if (a.Gx) g[p] += a.Gx[(size_t)w * NP * S::K + p * S::K + lm];
-            }
-            for (int tn = 0; tn < T; ++tn) {
-                float v[S::N1P];
-#pragma unroll
-                for (int n = 0; n < S::N1P; ++n) {
-                    v[n] = 0.f;
-#pragma unroll
-                    for (int p = n; p < NP; p += N1)
-                        if (n < N1) v[n] += al[tn * NP + p] * g[p];
+                g[p] = make_float2(co.x * gf[p * a.sl + l0] * Ain[p * S::K + k0],
+                                   co.y * gf[p * a.sl + l1] * Ain[p * S::K + k1]);
+                if (Gx) {
+                    g[p].x += nm.x * Gx[p * S::K + k0];
+                    g[p].y += nm.y * Gx[p * S::K + k1];
                 }
-                const float rs = lm != l * l + l ? kSqrt2 : 1.f;  // rows m != 0 carry sqrt2
-                float4* out = reinterpret_cast<float4*>(sGh + (size_t)(tn * S::K + lm) * S::N1P);
+            }
+            if (diag) {
+                for (int tn = 0; tn < T; ++tn) {
+                    const float* al = sAl + (tc * kFwdTypes + tn) * NP;
+                    float4* out = reinterpret_cast<float4*>(sGh + tn * S::GH + s * S::RF);
 #pragma unroll
-                for (int q = 0; q < S::N1P / 4; ++q)
-                    out[q] = make_float4(rs * v[4 * q], rs * v[4 * q + 1], rs * v[4 * q + 2], rs * v[4 * q + 3]);
+                    for (int q = 0; q < S::RF / 4; ++q) {
+                        float2 v[2];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            v[h] = make_float2(0.f, 0.f);
+                            const int n = 2 * q + h;
+                            if (n < N1) {
+#pragma unroll
+                                for (int p = n; p < NP; p += N1) v[h] = __ffma2_rn(make_float2(al[p], al[p]), g[p], v[h]);
+                            }
+                        }
+                        out[q] = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+                    }
+                }
+            } else {  // G transposed to [p][lm] in scratch
+                float* scr = sGh + T * S::GH;
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    if (s >= S::NZ || 2 * s + 1 <= L) scr[p * S::K + k1] = g[p].y;
+                    scr[p * S::K + k0] = g[p].x;
+                }
             }
         }
-        __syncwarp();
-    } else {
-        // G[p][lm] = 2 * 4pi/(2l+1) * dE/dfp[p][l] * A[p][lm], transposed into scr
-        const float* Ain = a.A + (size_t)w * NP * S::K;
-        const float* gf = a.gfp + (size_t)(s0 + w) * a.fp_stride + a.fp_off;
-        for (int lm = lane; lm < S::K; lm += 32) {
-            int l = 0;
-            while ((l + 1) * (l + 1) <= lm) ++l;
-            const float coef = l < a.nl2 ? 2.f * kPi4 / (float)(2 * l + 1) : 0.f;
-            const int lc = l < a.nl2 ? l : 0;
+    }
+    __syncwarp();
+    if (!diag) {
+        if (act) {
+            const float* scr = sGh + T * S::GH;
+            for (int idx = sub; idx < T * S::NS; idx += LPA) {
+                const int tn = idx / S::NS, s = idx - tn * S::NS;
+                int k0, k1;
+                if (s < S::NZ) {
+                    const int l1 = min(2 * s + 1, L);
+                    k0 = 4 * s * s + 2 * s;
+                    k1 = 2 * s + 1 <= L ? l1 * l1 + l1 : -1;
+                } else {
+                    int t = s - S::NZ, m = 1;
+                    for (; t >= L - m + 1; ++m) t -= L - m + 1;
+                    const int l = m + t;
+                    k0 = l * l + l + m;
+                    k1 = l * l + l - m;
+                }
+                const int* np_ = sNp + (size_t)(tc * T + tn) * N1 * kNz;
+                const float* nw = sNw + (size_t)(tc * T + tn) * N1 * kNz;
+                float* out = sGh + tn * S::GH + s * S::RF;
 #pragma unroll
-            for (int p = 0; p < NP; ++p) {  // lanes over lm: conflict-free [p][K] stores
-                float v = coef * gf[p * a.sl + lc] * Ain[p * S::K + lm];
-                if (a.Gx) v += a.Gx[(size_t)w * NP * S::K + p * S::K + lm];
-                scr[p * S::K + lm] = v;
-            }
-        }
-        __syncwarp();
-        // Gh[tn][lm][n] from the sparse fuse table of (tc, tn); lanes over lm read G rows
-        // without conflicts and write their Gh rows as float4
-        for (int idx = lane; idx < T * S::K; idx += 32) {
-            const int tn = idx / S::K, lm = idx - tn * S::K;
-            const int* np_ = sNp + (size_t)(tc * T + tn) * N1 * kNz;
-            const float* nw = sNw + (size_t)(tc * T + tn) * N1 * kNz;
-            float v[S::N1P];
-#pragma unroll
-            for (int n = 0; n < S::N1P; ++n) {
-                v[n] = 0.f;
-                if (n < N1) {
+                for (int n = 0; n < N1; ++n) {
+                    float vx = 0.f, vy = 0.f;
 #pragma unroll
                     for (int z = 0; z < kNz; ++z) {
                         const int pp = np_[n * kNz + z];
-                        if (pp >= 0) v[n] += nw[n * kNz + z] * scr[pp * S::K + lm];
+                        if (pp >= 0) {
+                            vx += nw[n * kNz + z] * scr[pp * S::K + k0];
+                            if (k1 >= 0) vy += nw[n * kNz + z] * scr[pp * S::K + k1];
+                        }
                     }
+                    *reinterpret_cast<float2*>(out + 2 * n) = make_float2(vx, vy);
                 }
             }
-            int l = 0;
-            while ((l + 1) * (l + 1) <= lm) ++l;
-            const float rs = lm != l * l + l ? kSqrt2 : 1.f;  // rows m != 0 carry sqrt2
-            float4* out = reinterpret_cast<float4*>(sGh + (size_t)idx * S::N1P);
-#pragma unroll
-            for (int q = 0; q < S::N1P / 4; ++q)
-                out[q] = make_float4(rs * v[4 * q], rs * v[4 * q + 1], rs * v[4 * q + 2], rs * v[4 * q + 3]);
         }
         __syncwarp();
     }
-    float* sP = scr;  // [NT][32], one Legendre column per lane
-    constexpr int H2 = S::N1P / 2;
-    for (int base = 0; base < cnt; base += 32) {
-        const int k = base + lane;
-        float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
-        float r = 1.f;
+    for (int base = 0; base < cmax; base += LPA) {
+        const int k = base + sub;
+        float4 d = make_float4(0.f, 0.f, 1.f, 0.f);
         bool valid = false;
+        float r = 1.f;
         if (k < cnt) {
             d = a.P.dx[(size_t)at * M + k];
             r = sqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
             valid = r < rc;
         }
         const int tn = valid ? __float_as_int(d.w) - 1 : 0;
-        const float u = r * irc, fc1 = 1.f - u * u, fc2 = fc1 * fc1, fc = valid ? fc2 * fc2 : 0.f;
-        const float x = 1.f - 2.f * u;
-        float Tn[S::N1P];
-        cheby_f<N1>(x, Tn);
+        const float ir = 1.f / r, x = d.x * ir, y = d.y * ir, z = d.z * ir;
+        const float u = r * irc, tx = 1.f - 2.f * u;
+        float Tn[N1];
+        cheby_f<N1>(tx, Tn);
+        float2 T2[N1], v2[N1];
 #pragma unroll
-        for (int n = N1; n < S::N1P; ++n) Tn[n] = 0.f;
-        const Angles an = angles_f(d.x, d.y, d.z, r);
+        for (int n = 0; n < N1; ++n) {
+            T2[n] = make_float2(Tn[n], Tn[n]);
+            v2[n] = make_float2(0.f, 0.f);
+        }
+        const float* gh = sGh + tn * S::GH;
+        float gx = 0.f, gy = 0.f, gz;
         {
-            float Pv[S::NT];
-            legendre_f<L>(an.ct, an.st, Pv);
+            float q0[L + 2], q1[L + 2];
+            monic_column<L, 0>(z, q0);
+            q0[L + 1] = 0.f;
+            q1[0] = 0.f;
+            if constexpr (L >= 1) monic_column<L, 1>(z, q1);
+            q1[L + 1] = 0.f;
+            float2 az = make_float2(0.f, 0.f);
 #pragma unroll
-            for (int q = 0; q < S::NT; ++q) sP[q * 32 + lane] = valid ? Pv[q] : 0.f;
+            for (int s = 0; s < S::NZ; ++s) {
+                const int l = 2 * s;
+                const float2 dy = gh_row<N1>(gh + s * S::RF, T2, make_float2(q0[l], q0[l + 1]), v2);
+                az = __ffma2_rn(make_float2((float)l * q1[l], (float)(l + 1) * q1[l + 1]), dy, az);
+            }
+            gz = az.x + az.y;
+            if constexpr (L >= 1) bwd_columns<L, N1, 1>(gh, T2, v2, x, y, z, q1, x, y, 1.f, 0.f, gx, gy, gz);
         }
-        __syncwarp();
-        float2 T2[H2], v2[H2];
-#pragma unroll
-        for (int h = 0; h < H2; ++h) {
-            T2[h] = make_float2(fc * Tn[2 * h], fc * Tn[2 * h + 1]);
-            v2[h] = make_float2(0.f, 0.f);
-        }
-        const float* gh = sGh + (size_t)tn * S::K * S::N1P;
-        // one Gh row: returns dY_lm and adds Gh[lm][n] * y into v.  Whole float4 groups of
-        // the N1 radial functions, then the remainder (the row's padding is never multiplied)
-        auto row = [&](int lm, float y) -> float {
-            const float4* gr = reinterpret_cast<const float4*>(gh + lm * S::N1P);
-            const float2 yy = make_float2(y, y);
-            float2 da = make_float2(0.f, 0.f), db = make_float2(0.f, 0.f);
-            constexpr int NQ = N1 / 4, NR = N1 - 4 * (N1 / 4);
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) {
-                const float4 g = gr[q];
-                const float2 ga = make_float2(g.x, g.y), gb = make_float2(g.z, g.w);
-                da = __ffma2_rn(T2[2 * q], ga, da);
-                db = __ffma2_rn(T2[2 * q + 1], gb, db);
-                v2[2 * q] = __ffma2_rn(ga, yy, v2[2 * q]);
-                v2[2 * q + 1] = __ffma2_rn(gb, yy, v2[2 * q + 1]);
-            }
-            if (NR >= 2) {
-                const float2 ga = reinterpret_cast<const float2*>(gr + NQ)[0];
-                da = __ffma2_rn(T2[2 * NQ], ga, da);
-                v2[2 * NQ] = __ffma2_rn(ga, yy, v2[2 * NQ]);
-            }
-            if (NR & 1) {
-                constexpr int n = N1 - 1;
-                const float g = gh[lm * S::N1P + n];
-                if (n & 1) {
-                    db.y = fmaf(T2[n >> 1].y, g, db.y);
-                    v2[n >> 1].y = fmaf(g, y, v2[n >> 1].y);
-                } else {
-                    db.x = fmaf(T2[n >> 1].x, g, db.x);
-                    v2[n >> 1].x = fmaf(g, y, v2[n >> 1].x);
-                }
-            }
-            return (da.x + db.x) + (da.y + db.y);
-        };
-        const float cp = an.cp, sp = an.sp;
-        float gth = 0.f, gph = 0.f;
-#pragma unroll
-        for (int l = 0; l <= L; ++l) {
-            const int c0 = l * l + l, tl = l * (l + 1) / 2;
-            const float p0 = sP[tl * 32 + lane];
-            const float p1 = l >= 1 ? sP[(tl + 1) * 32 + lane] : 0.f;
-            // m = 0: dP/dtheta = (dup P_{l,1} + ddn P_{l,1}) / 2 (P_{l,-1} = -P_{l,1})
-            gth += row(c0, p0) * (0.5f * (c_dup[tl] + c_ddn[tl]) * p1);
-            float cmm = 1.f, cmv = cp, smm = 0.f, smv = sp;
-            float pmm = p0, pmv = p1;
-#pragma unroll
-            for (int m = 1; m <= l; ++m) {
-                const int t = tl + m;
-                const float pmp = m + 1 <= l ? sP[(t + 1) * 32 + lane] : 0.f;
-                const float dpt = 0.5f * (c_dup[t] * pmp - c_ddn[t] * pmm);
-                const float yp = pmv * cmv, ym = pmv * smv;  // Y / sqrt2 (the Gh rows carry sqrt2)
-                const float dYp = row(c0 + m, yp);
-                const float dYm = row(c0 - m, ym);
-                gth += dpt * (dYp * cmv + dYm * smv);
-                gph += (float)m * (dYm * yp - dYp * ym);
-                const float cn = 2.f * cp * cmv - cmm, sn = 2.f * cp * smv - smm;
-                cmm = cmv; cmv = cn; smm = smv; smv = sn;
-                pmm = pmv; pmv = pmp;
-            }
-        }
-        __syncwarp();  // the Legendre columns are rewritten by the next batch
         if (k < cnt) {
             const size_t e = (size_t)at * M + k;
             float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
             if (valid) {
+                // radial part: -(1/r) d/dr of fc and of T_n (n U_{n-1} 2 / (r rc))
+                const float fc1 = 1.f - u * u, fc2 = fc1 * fc1, fc = fc2 * fc2;
                 const float fcg = 8.f * fc1 * fc2 * irc * irc;
-                float TG[N1], Tr[N1];  // T_n formed again: fc T_n went into the row products
-                cheby_grad_f<N1>(x, 2.f / (r * rc), TG);
-                cheby_f<N1>(x, Tr);
-                float dfc = 0.f, drn = 0.f;
+                float dfc = v2[0].x + v2[0].y, drn = 0.f, um1 = 1.f, um2 = 0.f;
 #pragma unroll
-                for (int n = 0; n < N1; ++n) {
-                    const float vn = (n & 1) ? v2[n >> 1].y : v2[n >> 1].x;
-                    dfc += vn * Tr[n];
-                    drn += vn * TG[n];
+                for (int n = 1; n < N1; ++n) {
+                    const float vn = v2[n].x + v2[n].y;
+                    dfc = fmaf(vn, Tn[n], dfc);
+                    drn = fmaf((float)n * vn, um1, drn);
+                    const float un = fmaf(2.f * tx, um1, -um2);
+                    um2 = um1;
+                    um1 = un;
                 }
-                const float gr = dfc * fcg + fc * drn;
-                const float ir = 1.f / r;
-                const float tpx = -an.ct * an.cp * ir, tpy = -an.ct * an.sp * ir, tpz = an.st * ir;
-                const float ppx = an.pole ? 0.f : an.sp / an.dxy, ppy = an.pole ? 0.f : -an.cp / an.dxy;
-                g.x = gr * d.x + gth * tpx + gph * ppx;
-                g.y = gr * d.y + gth * tpy + gph * ppy;
-                g.z = gr * d.z + gth * tpz;
+                const float gr = dfc * fcg + fc * (drn * (2.f * ir * irc));
+                // a neighbour on the z axis has no phi terms (basis_SphericalUtil.hpp:160-181):
+                // phi = 0 there, so the y component of the angular part is dropped
+                if (fmaxf(fabsf(d.x), fabsf(d.y)) < 8.f * 1.17549435e-38f) gy = 0.f;
+                const float f = fc * ir, un = fmaf(x, gx, fmaf(y, gy, z * gz));
+                g.x = fmaf(gr, d.x, f * fmaf(x, un, -gx));
+                g.y = fmaf(gr, d.y, f * fmaf(y, un, -gy));
+                g.z = fmaf(gr, d.z, f * fmaf(z, un, -gz));
             }
             if (a.accumulate) {
                 if (valid) {
@@ -1080,23 +1146,38 @@ cudaError_t launch_radial(const DescArgs& a, bool fwd, cudaStream_t st) {
     return launch_pdl(&k_radial_bwd<NP, N1, RB>, dim3(grid), dim3(32 * wpc), sm, st, a);
 }
 
-template <int L, int NP, int N1>
-cudaError_t launch_sph_bwd_n(const DescArgs& a, cudaStream_t st) {
+template <int L, int NP, int N1, int LPA>
+cudaError_t launch_sph_bwd_lanes(const DescArgs& a, cudaStream_t st) {
     using S = SphNShape<L, NP, N1>;
-    const int wpc = a.warps;
-    const int grid = (a.nmax + wpc - 1) / wpc;
-    const size_t nal = (a.fwd_alpha && a.T <= kFwdTypes) ? (size_t)a.T * kFwdTypes * NP : 0;
-    const size_t sm = sizeof(float) * (((size_t)2 * a.T * a.T * N1 * kNz + 3) / 4 * 4 + (nal + 3) / 4 * 4 +
-                                       (size_t)wpc * S::warp_floats(a.T));
+    constexpr int APW = 32 / LPA;
+    const bool diag = a.fwd_alpha && a.T <= kFwdTypes;
+    const size_t fixed = (4 * (size_t)S::NS + 3) / 4 * 4 +
+                         ((diag ? (size_t)a.T * kFwdTypes * NP : (size_t)2 * a.T * a.T * N1 * kNz) + 3) / 4 * 4;
+    int wpc = a.warps < kBwdWarps ? a.warps : kBwdWarps;
+    while (wpc > 1 && sizeof(float) * (fixed + (size_t)wpc * S::warp_floats(a.T, APW, diag)) > 227 * 1024) wpc >>= 1;
+    const size_t sm = sizeof(float) * (fixed + (size_t)wpc * S::warp_floats(a.T, APW, diag));
     if (sm > 227 * 1024) return cudaErrorInvalidValue;
+    const int grid = (a.nmax + wpc * APW - 1) / (wpc * APW);
     static int lim = 0;
     if ((int)sm > lim) {
         const cudaError_t e =
-            cudaFuncSetAttribute(k_sph_bwd_n<L, NP, N1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            cudaFuncSetAttribute(k_sph_bwd_n<L, NP, N1, LPA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
         lim = (int)sm;
     }
-    return launch_pdl(&k_sph_bwd_n<L, NP, N1>, dim3(grid), dim3(32 * wpc), sm, st, a);
+    return launch_pdl(&k_sph_bwd_n<L, NP, N1, LPA>, dim3(grid), dim3(32 * wpc), sm, st, a);
+}
+
+template <int L, int NP, int N1>
+cudaError_t launch_sph_bwd_n(const DescArgs& a, cudaStream_t st) {
+    using S = SphNShape<L, NP, N1>;
+    // Sixteen lanes per atom waste fewer lanes on the last neighbours of a row (40 neighbours:
+    // 48 lane slots instead of 64; 1M-atom glass, lmax 4: 1.76 against 2.58 ms) while the Gh of
+    // two atoms leaves shared memory for six CTAs; with larger Gh (lmax 6, three species: 12 KB)
+    // thirty-two are faster (1024-structure batch 1.96 against 2.05 ms).  Below 4096 atoms the
+    // SMs are not filled and the shorter walk of thirty-two lanes wins (33 atoms: 10 against 15 us).
+    if (a.nmax >= 4096 && 2 * sizeof(float) * a.T * S::GH <= 6400) return launch_sph_bwd_lanes<L, NP, N1, 16>(a, st);
+    return launch_sph_bwd_lanes<L, NP, N1, 32>(a, st);
 }
 
 template <int L, int NP, int N1>
@@ -1122,7 +1203,7 @@ cudaError_t launch_sph(const DescArgs& a, bool fwd, cudaStream_t st) {
     const int n = a.nmax;
     if (n <= 0) return cudaSuccess;
     if constexpr (RB == kRbNNAP) {   // the radial-space kernels are written for the NNAP radial functions
-        if (!fwd && a.nz_p && a.nz_w && N1 < NP) return launch_sph_bwd_n<L, NP, N1>(a, st);
+        if (!fwd && a.nz_p && a.nz_w && N1 <= NP) return launch_sph_bwd_n<L, NP, N1>(a, st);
         if (fwd && a.fwd_alpha && N1 < NP && a.T <= kFwdTypes) {
             if constexpr (SphTcShape<L, NP>::fits)
                 if (a.tc_sms > 0) return launch_sph_fwd_tc<L, NP, N1>(a, st);
@@ -1179,6 +1260,7 @@ cudaError_t launch_descriptor(int kind, int basis, int lmax, int np, int n1, con
         constexpr int RB_ = kRbNNAP;
         NNAP_RADIAL_SHAPES(R_CASE)
         NNAP_SPH_SHAPES(S_CASE)
+        NNAP_SPH_EVAL_SHAPES(S_CASE)
     } else if (basis == kRbNEP) {
         constexpr int RB_ = kRbNEP;
         NEP_RADIAL_SHAPES(R_CASE)

@@ -81,10 +81,14 @@ void upload_model(nnap_handle* h) {
             r.W.emplace_back();
             r.W.back().ensure(W.size());
             CK(cudaMemcpy(r.W.back().p, W.data(), W.size() * sizeof(float), cudaMemcpyHostToDevice));
+            // one channel per radial function (N1 == NP) and a cutoff well inside the neighbour
+            // cutoff after the first sub-basis: the channel-space kernels over compact rows win
+            const bool compact = s.kind == KIND_SPHERICAL && k > 0 && s.rcut <= 0.85 * m.rcut_max;
+            const bool rspace = s.kind == KIND_SPHERICAL && s.basis == kRbNNAP && (s.n1 < s.np || (s.n1 == s.np && !compact));
             // sparse columns for the radial-space backward
             std::vector<int> zp((size_t)T * T * s.n1 * kNz, -1);
             std::vector<float> zw(zp.size(), 0.f);
-            bool sparse = s.kind == KIND_SPHERICAL && s.n1 < s.np && s.basis == kRbNNAP;
+            bool sparse = rspace;
             for (int tc = r.t0; tc < r.t1 && sparse; ++tc)
                 for (int tn = 0; tn < T && sparse; ++tn)
                     for (int n = 0; n < s.n1 && sparse; ++n) {
@@ -124,7 +128,7 @@ void upload_model(nnap_handle* h) {
             // per-row scales for the radial-space forward
             {
                 std::vector<float> al((size_t)T * kFwdTypes * s.np, 0.f);
-                bool diag = s.kind == KIND_SPHERICAL && s.n1 < s.np && T <= kFwdTypes && s.basis == kRbNNAP;
+                bool diag = rspace && T <= kFwdTypes;
                 for (int tc = r.t0; tc < r.t1 && diag; ++tc)
                     for (int tn = 0; tn < T && diag; ++tn)
                         for (int p = 0; p < s.np && diag; ++p)
@@ -146,7 +150,7 @@ void upload_model(nnap_handle* h) {
             // well inside the neighbour cutoff scans compact rows (one such cutoff per model)
             {
                 const bool pspace = !sparse && !r.falpha.back().p;
-                bool use = s.kind == KIND_SPHERICAL && k > 0 && pspace && s.rcut <= 0.85 * m.rcut_max;
+                const bool use = compact && pspace;
                 if (use && h->sub_rc == 0.0) h->sub_rc = s.rcut;
                 r.use_sub.push_back(use && s.rcut == h->sub_rc);
             }

@@ -16,6 +16,8 @@ namespace {
 
 __constant__ float c_shA[91], c_shB[91], c_dup[91], c_ddn[91];
 __constant__ float c_diag[13], c_sub[13];
+// Factors of the monic harmonics (below): Y_{l,+-m} = c_shN[tri(l,m)] Q_lm(z) {Re, Im}(x + iy)^m.
+__constant__ float c_shN[91];
 
 // Recursion coefficients of the normalised associated Legendre functions for l <= 12.
 cudaError_t upload_sh_tables() {
@@ -30,6 +32,17 @@ cudaError_t upload_sh_tables() {
             up[t] = (float)sqrt((double)(l - m) * (l + m + 1));
             dn[t] = (float)sqrt((double)(l + m) * (l - m + 1));
         }
+    // sqrt2 (m > 0) (-1)^m sqrt((2l+1)/(4 pi) (l-m)!/(l+m)!) times the leading coefficient
+    // (2l-1)!!/(l-m)! of d^m P_l / dz^m
+    float nm[91] = {0};
+    for (int l = 0; l <= 12; ++l)
+        for (int m = 0; m <= l; ++m) {
+            double f = (2.0 * l + 1.0) / 12.566370614359172, c = 1.0;
+            for (int k = l - m + 1; k <= l + m; ++k) f /= k;
+            for (int k = 1; k <= l; ++k) c *= 2.0 * k - 1.0;
+            for (int k = 1; k <= l - m; ++k) c /= k;
+            nm[l * (l + 1) / 2 + m] = (float)((m & 1 ? -1.0 : 1.0) * sqrt(m ? 2.0 * f : f) * c);
+        }
     for (int m = 0; m <= 12; ++m) {
         dg[m] = m ? (float)sqrt(1.0 + 0.5 / m) : 0.f;
         sb[m] = (float)sqrt(2.0 * m + 3.0);
@@ -40,6 +53,7 @@ cudaError_t upload_sh_tables() {
     if ((e = cudaMemcpyToSymbol(c_dup, up, sizeof(up))) != cudaSuccess) return e;
     if ((e = cudaMemcpyToSymbol(c_ddn, dn, sizeof(dn))) != cudaSuccess) return e;
     if ((e = cudaMemcpyToSymbol(c_diag, dg, sizeof(dg))) != cudaSuccess) return e;
+    if ((e = cudaMemcpyToSymbol(c_shN, nm, sizeof(nm))) != cudaSuccess) return e;
     return cudaMemcpyToSymbol(c_sub, sb, sizeof(sb));
 }
 
@@ -124,6 +138,27 @@ __device__ __forceinline__ void legendre_f(float ct, float st, float* P) {
 #pragma unroll
         for (int l = m + 2; l <= L; ++l)
             P[tri(l, m)] = c_shA[tri(l, m)] * (ct * P[tri(l - 1, m)] + c_shB[tri(l, m)] * P[tri(l - 2, m)]);
+}
+
+// Monic harmonics of a unit vector (x, y, z).  With Q_lm(z) the m-th derivative of the
+// Legendre polynomial P_l scaled to leading coefficient one,
+//   Y_{l,m}  = N_lm Q_lm(z) Re (x + iy)^m,   Y_{l,-m} = N_lm Q_lm(z) Im (x + iy)^m,
+//   Q_mm = 1, Q_{m+1,m} = z, Q_lm = z Q_{l-1,m} - beta_lm Q_{l-2,m},
+//   beta_lm = ((l-1)^2 - m^2) / (4 (l-1)^2 - 1),   dQ_lm/dz = (l - m) Q_{l,m+1},
+// so no angle, trigonometric recurrence or division by sin(theta) is formed, a column of one m
+// takes two operations per entry, and the factors N_lm (c_shN) multiply per-atom sums instead
+// of every neighbour's harmonics.
+constexpr float leg_beta(int l, int m) {
+    return (float)(((double)(l - 1) * (l - 1) - (double)m * m) / (4.0 * (l - 1) * (l - 1) - 1.0));
+}
+
+// Column m: q[l] = Q_lm(z) for l = m .. L (other entries untouched).
+template <int L, int m>
+__device__ __forceinline__ void monic_column(float z, float* q) {
+    if (m <= L) q[m] = 1.f;
+    if (m + 1 <= L) q[m + 1] = z;
+#pragma unroll
+    for (int l = m + 2; l <= L; ++l) q[l] = fmaf(z, q[l - 1], -leg_beta(l, m) * q[l - 2]);
 }
 
 struct Angles {
