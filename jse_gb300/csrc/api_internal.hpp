@@ -31,8 +31,10 @@ __global__ void k_cell_order(const int*, int, const float4*, const float4*, floa
 __global__ void k_renumber(int*, int, const float4*, const float4*, const double*, const int*, const int*, float4*,
                            float4*, double*, int*, int*, int*);
 __global__ void k_unpermute(const double*, const int*, int, double*);
-__global__ void k_neighbors(const StructDev*, const int*, const double*, const float4*, const float4*, const float4*,
-                            const float4*, const int*, const int*, const int*, int, PairBufs, int*, int*);
+// Neighbour rows (k_neighbors); max_off: at least the stencil cells of every structure.
+cudaError_t launch_neighbors(const StructDev* S, const int* sid, const double* xw, const float4* xfc, const float4* xloc,
+                             const int* cell_of, const int* cell_start, const int* cell_atoms, int n, int max_off,
+                             int warps, int sms, const PairBufs& P, int* err, int* max_count, cudaStream_t st);
 __global__ void k_mirror(const StructDev*, const int*, PairBufs, int, int*);
 __global__ void k_type_hist(const int*, int, int, int*);
 __global__ void k_type_offsets(int*, int, int, int*);
@@ -164,7 +166,11 @@ struct Batch {
     int nstruct = 0, natoms = 0, ncells = 0;
     std::vector<StructDev> sd;
     std::vector<int> cb, ce, sc;
+    int max_off = 0;  // most stencil cells of a structure
 };
+
+// Stencil cells (cell offsets searched) of a structure.
+inline int stencil_cells(const StructDev& d) { return (2 * d.R[0] + 1) * (2 * d.R[1] + 1) * (2 * d.R[2] + 1); }
 
 struct Outputs {
     double *energy = nullptr, *energies = nullptr, *forces = nullptr, *virial = nullptr, *virials = nullptr;

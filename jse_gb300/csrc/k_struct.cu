@@ -152,14 +152,24 @@ __global__ void k_sort_cells(const int* __restrict__ cell_start, int ncells, int
 }
 
 // ----------------------------------------------------------------- neighbour rows
-// One warp per atom.  Candidate cells are visited in a fixed order; within a batch
-// of 32 cells the candidates are spread over the lanes, screened in FP32 against
-// rc^2 plus a rounding margin, and confirmed with the exact FP64 test.  Accepted
-// pairs are compacted in candidate order with a ballot, so rows are deterministic.
+// One warp per chunk of up to kNbAtoms consecutive cell-order positions.  The atoms of the
+// chunk that share a cell share its candidates: the stencil cells' ranges, image shifts and
+// pruning, and each window of 32 candidates (one per lane, shifted position in registers), are
+// formed once and screened in FP32 against every atom of the run (rc^2 plus a rounding margin).
+// Candidates that pass (about one in six) queue per atom in shared memory in candidate order
+// and take the exact test 32 at a time, so its lanes stay busy.  Accepted pairs are compacted
+// in candidate order with a ballot, so rows are deterministic and do not depend on the chunk.
 // Candidate positions are read from the cell-ordered copies xfc / xloc (k_cell_order), so
 // a lane's atom index and position loads are independent and a cell's candidates are
 // contiguous in memory.
+// Bound: instruction issue and its dependences (1145 warp instructions per atom at 24 warps per
+// SM, 53 % of the issue slots with 8 atoms per warp; one atom per warp, which set up its cells and looked up the cell
+// of each candidate for itself, took 2068 at 75 %).  Neighbour stage of the batch of 1024
+// structures 1.78 -> 1.40 ms, of the 1M-atom glass 3.05 -> 2.33 ms.
 constexpr int kNbMaxWarps = 8;  // warps per CTA are a launch parameter (2, 4 or 8)
+constexpr int kNbAtoms = 8;     // most atoms per warp
+constexpr int kNbQueue = 128;   // queued candidates per atom
+constexpr int kNbSpan = 4;      // most cells between the first and last atom of a run
 
 // floor(a / b) for b >= 1 and |a| < 2^22, from a float reciprocal of b and one correction
 // step (the float quotient is within one of the true one).
@@ -217,244 +227,382 @@ __global__ void k_unpermute(const double* __restrict__ in, const int* __restrict
     if (k < n) out[orig[k]] = in[k];
 }
 
-__global__ void __launch_bounds__(32 * kNbMaxWarps, 4)
-k_neighbors(const StructDev* __restrict__ S, const int* __restrict__ sid, const double* __restrict__ xw,
-            const float4* __restrict__ xf, const float4* __restrict__ xlo, const float4* __restrict__ xfc,
-            const float4* __restrict__ xloc, const int* __restrict__ cell_of, const int* __restrict__ cell_start,
-            const int* __restrict__ cell_atoms, int n, PairBufs P, int* __restrict__ err,
-            int* __restrict__ max_count) {
-    pdl_enter();
-    __shared__ int s_base[kNbMaxWarps][32];     // per cell slot: cell-order start minus candidate start
-    __shared__ int s_slot_at[kNbMaxWarps][32];  // cell slot starting at each position of a window
+// Shared memory of one warp; SLOTS stencil cells are held at a time (all of them where the
+// structure has at most SLOTS).
+template <int SLOTS, int NA>
+struct NbWarp {
     // per cell slot: the image shift's high parts and the packed image (one 16-byte load in
-    // the candidate loop), and the shift's low parts (the float-float test)
-    __shared__ float4 s_sh4[kNbMaxWarps][32];
-    __shared__ float s_flo[kNbMaxWarps][32][3];
-    __shared__ int s_acc[kNbMaxWarps][32];  // accepted entries per cell-offset group of the batch
-    __shared__ int s_qs[kNbMaxWarps][64];   // candidates passing the FP32 screen: cell slot,
-    __shared__ int s_qk[kNbMaxWarps][64];   // position in cell order
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int i = blockIdx.x * (blockDim.x >> 5) + w;
-    if (i >= n) return;
-    const StructDev& st = S[sid[i]];
-    const int M = P.M;
-    const int cl = cell_of[i] - st.c0;
-    const int ci0 = cl % st.nc[0], ci1 = (cl / st.nc[0]) % st.nc[1], ci2 = cl / (st.nc[0] * st.nc[1]);
-    const int wa = 2 * st.R[0] + 1, wb = 2 * st.R[1] + 1;
-    const int noff = wa * wb * (2 * st.R[2] + 1);
-    const float4 fi = xf[i];
-    const float4 li = xlo[i];
+    // the candidate loop), the shift's low parts (the float-float test), and the cell-order
+    // start minus the candidate start
+    float4 sh4[SLOTS];
+    float4 fi[NA], li[NA];  // the run's atoms
+    float4 box[2];                      // and their bounding box
+    float flo[SLOTS][3];
+    int base[32];
+    int slot_at[32];  // cell slot starting at each position of a window
+    int qn[NA], cnt[NA], last[NA];  // queued, accepted, last accepted group
+    int dx[NA];                                 // cells along a from the run's first
+    int qk[NA][kNbQueue];       // candidates passing the FP32 screen: position in cell order,
+    uint8_t qs[NA][kNbQueue];   // cell slot
+};
 
+// The exact test of the first qn queued candidates of atom q of the run (row i); accepted ones
+// are appended to the row.
+template <int SLOTS, int NA>
+__device__ __forceinline__ void nb_drain(NbWarp<SLOTS, NA>& sm, const StructDev& st, int q, int i, int o0, int noff,
+                                         int wa, int wu, const double* __restrict__ xw, const float4* __restrict__ xfc,
+                                         const float4* __restrict__ xloc, const int* __restrict__ cell_atoms,
+                                         const PairBufs& P, int lane) {
     const float rc2h = (float)st.rc2, rc2l = (float)(st.rc2 - (double)(float)st.rc2);
-    const float rc2_hi = st.rc2_hi;
     const float tol = 1e-10f * rc2h;  // float-float d^2 is accurate to ~1e-12 relative
-    int cnt = 0;
     const bool keep_groups = P.GS > noff;
-    for (int o0 = 0; o0 < noff; o0 += 32) {
-        const int o = o0 + lane;
-        const int cnt0 = cnt;
-        s_acc[w][lane] = 0;
-        int ccount = 0, cs = 0;
-        if (o < noff) {
-            const float inv_wa = __frcp_rn((float)wa), inv_wb = __frcp_rn((float)wb);
-            const float inv_nc0 = __frcp_rn((float)st.nc[0]), inv_nc1 = __frcp_rn((float)st.nc[1]),
-                        inv_nc2 = __frcp_rn((float)st.nc[2]);
-            const int oab = floor_div(o, wa, inv_wa), ocr = floor_div(oab, wb, inv_wb);
-            const int oa = o - oab * wa - st.R[0], ob = oab - ocr * wb - st.R[1], oc = ocr - st.R[2];
-            const int q0 = ci0 + oa, q1 = ci1 + ob, q2 = ci2 + oc;
-            const int na = floor_div(q0, st.nc[0], inv_nc0);
-            const int nb = floor_div(q1, st.nc[1], inv_nc1);
-            const int nc = floor_div(q2, st.nc[2], inv_nc2);
-            const int c0 = q0 - na * st.nc[0], c1 = q1 - nb * st.nc[1], c2 = q2 - nc * st.nc[2];
-            const int cid = st.c0 + c0 + st.nc[0] * (c1 + st.nc[1] * c2);
-            cs = cell_start[cid];
-            ccount = cell_start[cid + 1] - cs;
-            if (st.kind == 0) {
-                // orthogonal box: a lower bound of the distance from atom i to the target
-                // cell (unwrapped cell q spans [q, q+1) cell widths); cells beyond the screen
-                // bound (rc^2 plus its rounding margin) hold no neighbour and are skipped
-                const float wx = st.fa[0] / (float)st.nc[0], wy = st.fb[1] / (float)st.nc[1],
-                            wz = st.fc[2] / (float)st.nc[2];
-                const float gx = fmaxf(0.f, fmaxf((float)q0 * wx - fi.x, fi.x - (float)(q0 + 1) * wx));
-                const float gy = fmaxf(0.f, fmaxf((float)q1 * wy - fi.y, fi.y - (float)(q1 + 1) * wy));
-                const float gz = fmaxf(0.f, fmaxf((float)q2 * wz - fi.z, fi.z - (float)(q2 + 1) * wz));
-                if (gx * gx + gy * gy + gz * gz > rc2_hi) ccount = 0;
-            } else if (st.smin2 > 0.f) {
-                // skewed box: the gap in direct coordinates times the box's smallest
-                // singular value bounds the Cartesian distance from below (the atom's
-                // direct coordinates are formed here, so they hold no register in the
-                // candidate loop)
-                const int q[3] = {q0, q1, q2};
-                float g2 = 0.f;
+    const int M = P.M, qn = sm.qn[q];
+    const float4 fi = sm.fi[q], li = sm.li[q];
+    int cnt = sm.cnt[q], last = sm.last[q];
+    int* gs = P.gstart + (size_t)i * P.GS;
+    const int dx = SLOTS > 32 ? sm.dx[q] : 0;
+    const float inv_wu = __frcp_rn((float)wu);
+    for (int b = 0; b < qn; b += 32) {
+        bool acc = false;
+        int j = 0, slot = 0, g = 0;
+        uint32_t img = 0;
+        float fw = 0.f, ox = 0.f, oy = 0.f, oz = 0.f, lx = 0.f, ly = 0.f, lz = 0.f;
+        if (b + lane < qn) {
+            slot = sm.qs[q][b + lane];
+            const int kp = sm.qk[q][b + lane];
+            j = cell_atoms[kp];
+            const float4 s4 = sm.sh4[slot];
+            const float sh[3] = {s4.x, s4.y, s4.z};
+            img = __float_as_uint(s4.w);
+            const float4 fj = xfc[kp], lj = xloc[kp];
+            fw = fj.w;
+            // (x_j + shift) - x_i in float-float, then d^2 in float-float
+            float dh[3], dl[3];
+            const float ajh[3] = {fj.x, fj.y, fj.z}, ajl[3] = {lj.x, lj.y, lj.z};
+            const float aih[3] = {fi.x, fi.y, fi.z}, ail[3] = {li.x, li.y, li.z};
 #pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    const float ui = st.iv[d][0] * fi.x + st.iv[d][1] * fi.y + st.iv[d][2] * fi.z;
-                    const float inv_n = 1.f / (float)st.nc[d];
-                    const float g = fmaxf(0.f, fmaxf((float)q[d] * inv_n - ui, ui - (float)(q[d] + 1) * inv_n));
-                    g2 += g * g;
-                }
-                if (st.smin2 * g2 > rc2_hi) ccount = 0;
+            for (int d = 0; d < 3; ++d) {
+                float s1, e1, s2, e2;
+                two_sum(ajh[d], sh[d], s1, e1);
+                two_sum(s1, -aih[d], s2, e2);
+                const float lo = ((ajl[d] + sm.flo[slot][d]) - ail[d]) + (e1 + e2);
+                two_sum(s2, lo, dh[d], dl[d]);
             }
-
-            // the image shift as float-float on the FP32 pipe (the exact test forms the FP64
-            // shift itself); the zero image has an exactly zero shift
-            float hi[3], lo[3];
-            image_shift_ff(st, na, nb, nc, hi, lo);
-            s_sh4[w][lane] = make_float4(hi[0], hi[1], hi[2], __uint_as_float(pack_img(na, nb, nc)));
+            float d2h = 0.f, d2l = 0.f;
 #pragma unroll
-            for (int d = 0; d < 3; ++d) s_flo[w][lane][d] = lo[d];
-        }
-        int incl = ccount;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            int u = __shfl_up_sync(0xffffffffu, incl, d);
-            if (lane >= d) incl += u;
-        }
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        const int before = incl - ccount;  // candidates of the earlier cell slots
-        s_base[w][lane] = cs - before;
-        __syncwarp();
-        // Candidates are screened 32 at a time in FP32; the ones that pass (about one in four
-        // or five) queue in candidate order in shared memory and take the exact test 32 at a
-        // time, so its lanes stay busy.  Accepted entries keep candidate order.
-        int qn = 0;  // queued candidates (warp-uniform)
-        auto exact_batch = [&](int k) {  // the first k queued candidates
-            bool acc = false;
-            int j = 0, slot = 0;
-            uint32_t img = 0;
-            float4 fj = make_float4(0.f, 0.f, 0.f, 0.f);
-            float ox = 0.f, oy = 0.f, oz = 0.f, lx = 0.f, ly = 0.f, lz = 0.f;
-            if (lane < k) {
-                slot = s_qs[w][lane];
-                const int kp = s_qk[w][lane];
-                j = cell_atoms[kp];
-                const float4 s4 = s_sh4[w][slot];
-                const float sh[3] = {s4.x, s4.y, s4.z};
-                img = __float_as_uint(s4.w);
-                fj = xfc[kp];
-                const float4 lj = xloc[kp];
-                // (x_j + shift) - x_i in float-float, then d^2 in float-float
-                float dh[3], dl[3];
-                const float ajh[3] = {fj.x, fj.y, fj.z}, ajl[3] = {lj.x, lj.y, lj.z};
-                const float aih[3] = {fi.x, fi.y, fi.z}, ail[3] = {li.x, li.y, li.z};
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    float s1, e1, s2, e2;
-                    two_sum(ajh[d], sh[d], s1, e1);
-                    two_sum(s1, -aih[d], s2, e2);
-                    const float lo = ((ajl[d] + s_flo[w][slot][d]) - ail[d]) + (e1 + e2);
-                    two_sum(s2, lo, dh[d], dl[d]);
-                }
-                float d2h = 0.f, d2l = 0.f;
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    ff_acc_prod(d2h, d2l, dh[d], dh[d]);
-                    d2l += 2.f * dh[d] * dl[d];
-                }
-                const float diff = (d2h - rc2h) + (d2l - rc2l);
-                if (fabsf(diff) > tol) {
-                    acc = diff < 0.f;
-                } else {  // within 1e-10 of the cutoff: the exact FP64 test
-                    int na, nb, nc;
-                    unpack_img(img, na, nb, nc);
-                    double sh[3] = {0.0, 0.0, 0.0};
-                    if (na | nb | nc) image_shift(st, na, nb, nc, sh);
-                    const double dxv = ds(da(xw[3 * j], sh[0]), xw[3 * i]);
-                    const double dyv = ds(da(xw[3 * j + 1], sh[1]), xw[3 * i + 1]);
-                    const double dzv = ds(da(xw[3 * j + 2], sh[2]), xw[3 * i + 2]);
-                    acc = da(da(dm(dxv, dxv), dm(dyv, dyv)), dm(dzv, dzv)) < st.rc2;
-                }
-                if (j == i && img == pack_img(0, 0, 0)) acc = false;  // the atom itself
-                two_sum(dh[0], dl[0], ox, lx);
-                two_sum(dh[1], dl[1], oy, ly);
-                two_sum(dh[2], dl[2], oz, lz);
+            for (int d = 0; d < 3; ++d) {
+                ff_acc_prod(d2h, d2l, dh[d], dh[d]);
+                d2l += 2.f * dh[d] * dl[d];
             }
-            const unsigned m = __ballot_sync(0xffffffffu, acc);
-            if (acc) {
-                const int pos = cnt + __popc(m & ((1u << lane) - 1u));
-                if (pos < M) {
-                    const size_t e = (size_t)i * M + pos;
-                    P.key[e] = pair_key(j, img);
-                    P.dx[e] = make_float4(ox, oy, oz, fj.w);
-                    if (P.dxlo) P.dxlo[e] = make_float4(lx, ly, lz, 0.f);
-                    P.grp[e] = (uint16_t)(o0 + slot);
-                }
-                if (keep_groups) atomicAdd(&s_acc[w][slot], 1);
+            const float diff = (d2h - rc2h) + (d2l - rc2l);
+            if (fabsf(diff) > tol) {
+                acc = diff < 0.f;
+            } else {  // within 1e-10 of the cutoff: the exact FP64 test
+                int na, nb, nc;
+                unpack_img(img, na, nb, nc);
+                double sd[3] = {0.0, 0.0, 0.0};
+                if (na | nb | nc) image_shift(st, na, nb, nc, sd);
+                const double dxv = ds(da(xw[3 * (size_t)j], sd[0]), xw[3 * (size_t)i]);
+                const double dyv = ds(da(xw[3 * (size_t)j + 1], sd[1]), xw[3 * (size_t)i + 1]);
+                const double dzv = ds(da(xw[3 * (size_t)j + 2], sd[2]), xw[3 * (size_t)i + 2]);
+                acc = da(da(dm(dxv, dxv), dm(dyv, dyv)), dm(dzv, dzv)) < st.rc2;
             }
-            cnt += __popc(m);
-        };
-        // The cell slot of candidate cidx: the last nonempty slot starting at or before it.
-        // Per window of 32 candidates the starting positions form a bit mask (one OR
-        // reduction); a lane takes the highest start at or below its position, or the slot
-        // that ran into the window from the one before.
-        int carry = 0;
-        for (int cb = 0; cb < total; cb += 32) {
-            const int cidx = cb + lane;
-            const bool starts = ccount > 0 && before >= cb && before < cb + 32;
-            const unsigned smask = __reduce_or_sync(0xffffffffu, starts ? 1u << (before - cb) : 0u);
-            if (starts) s_slot_at[w][before - cb] = lane;
-            __syncwarp();
-            const unsigned mine = smask & (0xffffffffu >> (31 - lane));
-            const int slot = mine ? s_slot_at[w][31 - __clz(mine)] : carry;
-            carry = __shfl_sync(0xffffffffu, slot, 31);
-            // the screen reads only the candidate's cell-order position; its atom index is
-            // loaded by the exact test, which also drops the atom itself (zero image)
-            bool pass = false;
-            int kp = 0;
-            if (cidx < total) {
-                kp = s_base[w][slot] + cidx;
-                const float4 fj = xfc[kp];
-                const float4 sh = s_sh4[w][slot];
-                const float fx = (fj.x + sh.x) - fi.x;
-                const float fy = (fj.y + sh.y) - fi.y;
-                const float fz = (fj.z + sh.z) - fi.z;
-                pass = fx * fx + fy * fy + fz * fz < rc2_hi;
-            }
-            const unsigned m = __ballot_sync(0xffffffffu, pass);
-            if (pass) {
-                const int q = qn + __popc(m & ((1u << lane) - 1u));
-                s_qs[w][q] = slot;
-                s_qk[w][q] = kp;
-            }
-            qn += __popc(m);
-            __syncwarp();
-            if (qn >= 32) {
-                exact_batch(32);
-                // move the overflow (at most 31 entries) to the front of the queue
-                int rs = 0, rk = 0;
-                if (lane < qn - 32) {
-                    rs = s_qs[w][32 + lane];
-                    rk = s_qk[w][32 + lane];
-                }
-                __syncwarp();
-                if (lane < qn - 32) {
-                    s_qs[w][lane] = rs;
-                    s_qk[w][lane] = rk;
-                }
-                qn -= 32;
-                __syncwarp();
+            if (j == i && img == pack_img(0, 0, 0)) acc = false;  // the atom itself
+            two_sum(dh[0], dl[0], ox, lx);
+            two_sum(dh[1], dl[1], oy, ly);
+            two_sum(dh[2], dl[2], oz, lz);
+            g = o0 + slot;
+            if (SLOTS > 32) {  // the cell's offset from this atom's own cell
+                const int rest = floor_div(g, wu, inv_wu), oa = g - rest * wu - dx;
+                if (oa < 0 || oa >= wa) acc = false;
+                g = oa + wa * rest;
             }
         }
-        if (qn > 0) exact_batch(qn);
-        __syncwarp();
-        if (keep_groups) {  // start of each group of this batch: cnt0 + accepted entries of earlier groups
-            const int a = s_acc[w][lane];
-            int incl2 = a;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, incl2, d);
-                if (lane >= d) incl2 += u;
+        const unsigned m = __ballot_sync(0xffffffffu, acc);
+        const unsigned lower = m & ((1u << lane) - 1u);
+        const int gp = __shfl_sync(0xffffffffu, g, lower ? 31 - __clz(lower) : 0);
+        if (acc) {
+            const int pos = cnt + __popc(lower);
+            if (pos < M) {
+                const size_t e = (size_t)i * M + pos;
+                P.key[e] = pair_key(j, img);
+                P.dx[e] = make_float4(ox, oy, oz, fw);
+                if (P.dxlo) P.dxlo[e] = make_float4(lx, ly, lz, 0.f);
+                P.grp[e] = (uint16_t)g;
             }
-            if (o < noff) P.gstart[(size_t)i * P.GS + o] = cnt0 + incl2 - a;
+            // the groups after the last accepted entry's, up to this one's, start here
+            if (keep_groups)
+                for (int o = (lower ? gp : last) + 1; o <= g; ++o) gs[o] = pos;
         }
-        __syncwarp();
+        if (m) last = __shfl_sync(0xffffffffu, g, 31 - __clz(m));
+        cnt += __popc(m);
     }
+    __syncwarp();
     if (lane == 0) {
-        if (keep_groups) P.gstart[(size_t)i * P.GS + noff] = cnt;
-        P.count[i] = cnt;
-        if (cnt > M) atomicOr(err, ERRBIT_CAPACITY);
-        atomicMax(max_count, cnt);
+        sm.cnt[q] = cnt;
+        sm.last[q] = last;
+        sm.qn[q] = 0;
     }
+    __syncwarp();
+}
+
+// NA cell-order positions per warp.
+template <int SLOTS, int NA>
+__global__ void __launch_bounds__(32 * kNbMaxWarps, NA == 1 ? 4 : 3)
+k_neighbors(const StructDev* __restrict__ S, const int* __restrict__ sid, const double* __restrict__ xw,
+            const float4* __restrict__ xfc, const float4* __restrict__ xloc, const int* __restrict__ cell_of,
+            const int* __restrict__ cell_start, const int* __restrict__ cell_atoms, int n, PairBufs P,
+            int* __restrict__ err, int* __restrict__ max_count) {
+    pdl_enter();
+    extern __shared__ __align__(16) uint8_t nb_smem[];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    NbWarp<SLOTS, NA>& sm = reinterpret_cast<NbWarp<SLOTS, NA>*>(nb_smem)[w];
+    const int k0 = (blockIdx.x * (blockDim.x >> 5) + w) * NA;
+    const int k1 = min(n, k0 + NA);
+    int most = 0;
+    for (int kr = k0; kr < k1;) {
+        // the run [kr, kr + A): chunk positions in one cell; where cells are half the cutoff wide
+        // and hold a few atoms each (SLOTS > 32), in cells of one row along a, whose stencils
+        // overlap: candidates come in the same order for each of them
+        const int mine = kr + (lane & (NA - 1));
+        const int ia = cell_atoms[min(mine, k1 - 1)];
+        const int cell = cell_of[ia];
+        const int cell0 = __shfl_sync(0xffffffffu, cell, 0);
+        const int s0 = sid[__shfl_sync(0xffffffffu, ia, 0)];
+        const StructDev& st = S[s0];
+        bool in = cell == cell0;
+        if (SLOTS > 32)
+            in = cell - cell0 <= kNbSpan && sid[ia] == s0 && (cell - st.c0) / st.nc[0] == (cell0 - st.c0) / st.nc[0];
+        const unsigned same = __ballot_sync(0xffffffffu, lane < NA && mine < k1 && in);
+        const int A = __ffs(~same) - 1;  // atoms of a cell, and cells of a row, are contiguous
+        const int span = SLOTS > 32 ? __shfl_sync(0xffffffffu, cell, A - 1) - cell0 : 0;
+        const int kc = kr + min((int)(lane & (NA - 1)), A - 1);
+        const float4 f = xfc[kc], lo4 = xloc[kc];
+        __syncwarp();
+        if (lane < NA) {
+            sm.fi[lane] = f;
+            sm.li[lane] = lo4;
+            sm.qn[lane] = 0;
+            sm.cnt[lane] = 0;
+            sm.last[lane] = -1;
+            if (SLOTS > 32) sm.dx[lane] = cell - cell0;
+        }
+        // bounding box of the run's atoms (Cartesian, or direct coordinates in a skewed box)
+        float bl[3], bh[3];
+        if (st.kind == 0) {
+            bl[0] = f.x; bl[1] = f.y; bl[2] = f.z;
+        } else {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) bl[d] = st.iv[d][0] * f.x + st.iv[d][1] * f.y + st.iv[d][2] * f.z;
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            bh[d] = bl[d];
+#pragma unroll
+            for (int o = NA / 2; o > 0; o >>= 1) {
+                bl[d] = fminf(bl[d], __shfl_xor_sync(0xffffffffu, bl[d], o));
+                bh[d] = fmaxf(bh[d], __shfl_xor_sync(0xffffffffu, bh[d], o));
+            }
+        }
+        __syncwarp();
+        if (lane == 0) {
+            sm.box[0] = make_float4(bl[0], bl[1], bl[2], 0.f);
+            sm.box[1] = make_float4(bh[0], bh[1], bh[2], 0.f);
+        }
+        __syncwarp();
+        const int cl = cell0 - st.c0;
+        const int ci0 = cl % st.nc[0], ci1 = (cl / st.nc[0]) % st.nc[1], ci2 = cl / (st.nc[0] * st.nc[1]);
+        const int wa = 2 * st.R[0] + 1, wb = 2 * st.R[1] + 1;
+        const int noff = wa * wb * (2 * st.R[2] + 1);
+        const int wu = wa + span, nun = wu * wb * (2 * st.R[2] + 1);  // the run's stencil
+        const float rc2_hi = st.rc2_hi;
+        for (int o0 = 0; o0 < nun; o0 += SLOTS) {
+            for (int w0 = 0; w0 < SLOTS && o0 + w0 < nun; w0 += 32) {
+                const int o = o0 + w0 + lane;
+                int ccount = 0, cs = 0;
+                if (o < nun) {
+                    const float inv_wu = __frcp_rn((float)wu), inv_wb = __frcp_rn((float)wb);
+                    const float inv_nc0 = __frcp_rn((float)st.nc[0]), inv_nc1 = __frcp_rn((float)st.nc[1]),
+                                inv_nc2 = __frcp_rn((float)st.nc[2]);
+                    const int oab = floor_div(o, wu, inv_wu), ocr = floor_div(oab, wb, inv_wb);
+                    const int oa = o - oab * wu - st.R[0], ob = oab - ocr * wb - st.R[1], oc = ocr - st.R[2];
+                    const int q0 = ci0 + oa, q1 = ci1 + ob, q2 = ci2 + oc;
+                    const int na = floor_div(q0, st.nc[0], inv_nc0);
+                    const int nb = floor_div(q1, st.nc[1], inv_nc1);
+                    const int nc = floor_div(q2, st.nc[2], inv_nc2);
+                    const int c0 = q0 - na * st.nc[0], c1 = q1 - nb * st.nc[1], c2 = q2 - nc * st.nc[2];
+                    const int cid = st.c0 + c0 + st.nc[0] * (c1 + st.nc[1] * c2);
+                    cs = cell_start[cid];
+                    ccount = cell_start[cid + 1] - cs;
+                    const int q[3] = {q0, q1, q2};
+                    const float4 b0 = sm.box[0], b1 = sm.box[1];
+                    const float bl[3] = {b0.x, b0.y, b0.z}, bh[3] = {b1.x, b1.y, b1.z};
+                    if (st.kind == 0) {
+                        // orthogonal box: a lower bound of the distance from the run's bounding box
+                        // to the target cell (unwrapped cell q spans [q, q+1) cell widths); cells
+                        // beyond the screen bound (rc^2 plus its rounding margin) hold no neighbour
+                        const float wd[3] = {st.fa[0] / (float)st.nc[0], st.fb[1] / (float)st.nc[1],
+                                             st.fc[2] / (float)st.nc[2]};
+                        float g2 = 0.f;
+#pragma unroll
+                        for (int d = 0; d < 3; ++d) {
+                            const float g =
+                                fmaxf(0.f, fmaxf((float)q[d] * wd[d] - bh[d], bl[d] - (float)(q[d] + 1) * wd[d]));
+                            g2 += g * g;
+                        }
+                        if (g2 > rc2_hi) ccount = 0;
+                    } else if (st.smin2 > 0.f) {
+                        // skewed box: the gap in direct coordinates times the box's smallest
+                        // singular value bounds the Cartesian distance from below
+                        float g2 = 0.f;
+#pragma unroll
+                        for (int d = 0; d < 3; ++d) {
+                            const float inv_n = 1.f / (float)st.nc[d];
+                            const float g =
+                                fmaxf(0.f, fmaxf((float)q[d] * inv_n - bh[d], bl[d] - (float)(q[d] + 1) * inv_n));
+                            g2 += g * g;
+                        }
+                        if (st.smin2 * g2 > rc2_hi) ccount = 0;
+                    }
+                    // the image shift as float-float on the FP32 pipe (the exact test forms the FP64
+                    // shift itself); the zero image has an exactly zero shift
+                    float hi[3], lo[3];
+                    image_shift_ff(st, na, nb, nc, hi, lo);
+                    sm.sh4[w0 + lane] = make_float4(hi[0], hi[1], hi[2], __uint_as_float(pack_img(na, nb, nc)));
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) sm.flo[w0 + lane][d] = lo[d];
+                }
+                int incl = ccount;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    int u = __shfl_up_sync(0xffffffffu, incl, d);
+                    if (lane >= d) incl += u;
+                }
+                const int total = __shfl_sync(0xffffffffu, incl, 31);
+                const int before = incl - ccount;  // candidates of the earlier cell slots
+                sm.base[lane] = cs - before;
+                __syncwarp();
+                // The cell slot of candidate cidx: the last nonempty slot starting at or before it.
+                // Per window of 32 candidates the starting positions form a bit mask (one OR
+                // reduction); a lane takes the highest start at or below its position, or the slot
+                // that ran into the window from the one before.
+                int carry = 0, cb = 0;
+                const bool last = w0 + 32 >= SLOTS || o0 + w0 + 32 >= nun;
+                do {
+                    bool full = false;
+                    // the run's positions, read again after a drain: registers are not held over it
+                    float ax[NA], ay[NA], az[NA];
+                    int qn[NA];
+#pragma unroll
+                    for (int q = 0; q < NA; ++q) {
+                        const float4 v = sm.fi[q];
+                        ax[q] = v.x; ay[q] = v.y; az[q] = v.z;
+                        qn[q] = sm.qn[q];
+                    }
+                    for (; cb < total && !full; cb += 32) {
+                        const int cidx = cb + lane;
+                        const bool starts = ccount > 0 && before >= cb && before < cb + 32;
+                        const unsigned smask = __reduce_or_sync(0xffffffffu, starts ? 1u << (before - cb) : 0u);
+                        if (starts) sm.slot_at[before - cb] = lane;
+                        __syncwarp();
+                        const unsigned below = smask & (0xffffffffu >> (31 - lane));
+                        const int slot = below ? sm.slot_at[31 - __clz(below)] : carry;
+                        carry = __shfl_sync(0xffffffffu, slot, 31);
+                        // the screen reads only the candidate's cell-order position; its atom index is
+                        // loaded by the exact test, which also drops the atom itself (zero image)
+                        int kp = 0;
+                        float px = 3e38f, py = 0.f, pz = 0.f;  // no candidate: outside every cutoff
+                        if (cidx < total) {
+                            kp = sm.base[slot] + cidx;
+                            const float4 fj = xfc[kp];
+                            const float4 sh = sm.sh4[w0 + slot];
+                            px = fj.x + sh.x;
+                            py = fj.y + sh.y;
+                            pz = fj.z + sh.z;
+                        }
+#pragma unroll
+                        for (int q = 0; q < NA; ++q) {
+                            if (q < A) {
+                                const float fx = px - ax[q], fy = py - ay[q], fz = pz - az[q];
+                                const bool pass = fx * fx + fy * fy + fz * fz < rc2_hi;
+                                const unsigned m = __ballot_sync(0xffffffffu, pass);
+                                if (pass) {
+                                    const int at = qn[q] + __popc(m & ((1u << lane) - 1u));
+                                    sm.qk[q][at] = kp;
+                                    sm.qs[q][at] = (uint8_t)(w0 + slot);
+                                }
+                                qn[q] += __popc(m);
+                                full = full || qn[q] > kNbQueue - 32;
+                            }
+                        }
+                    }
+                    __syncwarp();
+                    if (lane == 0) {
+#pragma unroll
+                        for (int q = 0; q < NA; ++q) sm.qn[q] = qn[q];
+                    }
+                    __syncwarp();
+                    if (full || last)  // warp-uniform: every queue through the exact test
+                        for (int q = 0; q < A; ++q)
+                            nb_drain<SLOTS, NA>(sm, st, q, cell_atoms[kr + q], o0, noff, wa, wu, xw, xfc, xloc, cell_atoms, P, lane);
+                } while (cb < total);
+                __syncwarp();
+            }
+        }
+        if (P.GS > noff)
+            for (int q = 0; q < A; ++q) {
+                const int cnt = sm.cnt[q];
+                int* gs = P.gstart + (size_t)cell_atoms[kr + q] * P.GS;
+                for (int o = sm.last[q] + 1 + lane; o <= noff; o += 32) gs[o] = cnt;
+            }
+        if (lane < A) {
+            const int cnt = sm.cnt[lane];
+            P.count[ia] = cnt;
+            if (cnt > P.M) atomicOr(err, ERRBIT_CAPACITY);
+            most = max(most, cnt);
+        }
+        kr += A;
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0 && most > 0) atomicMax(max_count, most);
+}
+
+// Stencil cells held at a time and atoms per warp as template arguments of one launch.
+template <int SLOTS, int NA>
+static cudaError_t launch_nb(const StructDev* S, const int* sid, const double* xw, const float4* xfc, const float4* xloc,
+                             const int* cell_of, const int* cell_start, const int* cell_atoms, int n, int warps,
+                             const PairBufs& P, int* err, int* max_count, cudaStream_t st) {
+    const size_t smem = warps * sizeof(NbWarp<SLOTS, NA>);
+    if (smem > 48 * 1024) {
+        const cudaError_t e =
+            cudaFuncSetAttribute(k_neighbors<SLOTS, NA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    return launch_pdl(k_neighbors<SLOTS, NA>, dim3((unsigned)((n + warps * NA - 1) / (warps * NA))), dim3(32 * warps), smem,
+                      st, S, sid, xw, xfc, xloc, cell_of, cell_start, cell_atoms, n, P, err, max_count);
+}
+
+cudaError_t launch_neighbors(const StructDev* S, const int* sid, const double* xw, const float4* xfc, const float4* xloc,
+                             const int* cell_of, const int* cell_start, const int* cell_atoms, int n, int max_off,
+                             int warps, int sms, const PairBufs& P, int* err, int* max_count, cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
+    // atoms per warp: 8 where that leaves each SM 48 warps, two rounds of the resident ones,
+    // halved until it does.  The stage with 1, 2, 4 and 8 atoms per warp: 4000 atoms 63, 66, 73,
+    // 83 us; 25000 atoms 122, 122, 124, 131; 32000 atoms 141, 136, 130, 137 (half-width cells
+    // 258, 230, 219, 244); 1M atoms 3163, 2858, 2497, 2293
+    int chunk = kNbAtoms;
+    while (chunk > 1 && n < chunk * 48 * sms) chunk >>= 1;
+    const bool wide = max_off > 32;
+#define NB_CASE(N_)                                                                                                     \
+    if (chunk == N_)                                                                                                    \
+        return wide ? launch_nb<128, N_>(S, sid, xw, xfc, xloc, cell_of, cell_start, cell_atoms, n, warps, P, err,      \
+                                         max_count, st)                                                                 \
+                    : launch_nb<32, N_>(S, sid, xw, xfc, xloc, cell_of, cell_start, cell_atoms, n, warps, P, err,       \
+                                        max_count, st);
+    NB_CASE(8) NB_CASE(4) NB_CASE(2)
+    return wide ? launch_nb<128, 1>(S, sid, xw, xfc, xloc, cell_of, cell_start, cell_atoms, n, warps, P, err, max_count, st)
+                : launch_nb<32, 1>(S, sid, xw, xfc, xloc, cell_of, cell_start, cell_atoms, n, warps, P, err, max_count, st);
+#undef NB_CASE
 }
 
 // Mirror index: for entry (i -> j, image n) the position of (j -> i, image -n) in j's row.

@@ -392,6 +392,7 @@ const Batch& plan_batch(nnap_handle* h, int nstruct, const int* natoms, const in
         if (natoms[s] < 0) throw ApiFail(NNAP_ERR_ARG, "negative atom count");
         StructDev d = make_struct(kinds[s], boxes + 9 * s, rc, a0, natoms[s], c0);
         B.sd.push_back(d);
+        B.max_off = std::max(B.max_off, stencil_cells(d));
         for (int b = 0; b < natoms[s]; b += kRedChunk) {
             B.cb.push_back(a0 + b);
             B.ce.push_back(a0 + std::min(natoms[s], b + kRedChunk));
@@ -513,9 +514,7 @@ void prepare_layout(nnap_handle* h, const Batch& B) {
     if (h->M == 0) h->M = initial_capacity(B, h->model.rcut_max);
     ensure_work(h, n, B.nstruct, B.ncells, nchunks);
     // group starts of the neighbour rows, for the mirror search (kept up to 127 offset groups)
-    int gs = 0;
-    for (auto& d : B.sd) gs = std::max(gs, (2 * d.R[0] + 1) * (2 * d.R[1] + 1) * (2 * d.R[2] + 1) + 1);
-    h->GS = gs <= 128 ? gs : 0;
+    h->GS = B.max_off + 1 <= 128 ? B.max_off + 1 : 0;
     if (h->GS) h->gstart.ensure((size_t)std::max(n, 1) * h->GS);
     if (h->h_sdev_cap < (size_t)B.nstruct) {
         if (h->h_sdev) cudaFreeHost(h->h_sdev);
@@ -561,15 +560,15 @@ void enqueue_neighbors(nnap_handle* h, const Batch& B, const double* d_x, const 
             CK(launch_pdl(k_renumber, dim3((n + 255) / 256), dim3(256), 0, st, h->cell_atoms.p, n, h->xf.p, h->xlo.p,
                           h->xw.p, h->cell_of.p, d_type, h->xfc.p, h->xloc.p, h->xw2.p, h->cell_of2.p, h->type2.p,
                           h->orig.p));
-            CK(launch_pdl(k_neighbors, dim3((n + nw - 1) / nw), dim3(32 * nw), 0, st, h->sdev.p, h->sid.p, h->xw2.p,
-                          h->xfc.p, h->xloc.p, h->xfc.p, h->xloc.p, h->cell_of2.p, h->cell_start.p, h->cell_atoms.p,
-                          n, pair_bufs(h), h->status.p, h->status.p + 1));
+            CK(launch_neighbors(h->sdev.p, h->sid.p, h->xw2.p, h->xfc.p, h->xloc.p, h->cell_of2.p, h->cell_start.p,
+                                h->cell_atoms.p, n, B.max_off, nw, h->sm_count, pair_bufs(h), h->status.p, h->status.p + 1,
+                                st));
         } else {
             CK(launch_pdl(k_cell_order, dim3((n + 255) / 256), dim3(256), 0, st, h->cell_atoms.p, n, h->xf.p, h->xlo.p,
                           h->xfc.p, h->xloc.p));
-            CK(launch_pdl(k_neighbors, dim3((n + nw - 1) / nw), dim3(32 * nw), 0, st, h->sdev.p, h->sid.p, h->xw.p,
-                          h->xf.p, h->xlo.p, h->xfc.p, h->xloc.p, h->cell_of.p, h->cell_start.p, h->cell_atoms.p, n,
-                          pair_bufs(h), h->status.p, h->status.p + 1));
+            CK(launch_neighbors(h->sdev.p, h->sid.p, h->xw.p, h->xfc.p, h->xloc.p, h->cell_of.p, h->cell_start.p,
+                                h->cell_atoms.p, n, B.max_off, nw, h->sm_count, pair_bufs(h), h->status.p, h->status.p + 1,
+                                st));
         }
         h->launches += 4;
     }

@@ -133,8 +133,15 @@ extern "C" int nnap_neighbor_counts_noalloc(int natoms, const double* d_x, const
         P.M = 0;  // count only: no pair rows are written
         P.count = d_counts;
         k_cell_order<<<(natoms + 255) / 256, 256, 0, st>>>(cell_atoms, natoms, xf, xlo, xfc, xloc);
-        k_neighbors<<<(natoms + 3) / 4, 128, 0, st>>>(sdev, sid, xw, xf, xlo, xfc, xloc, cell_of, cell_start, cell_atoms,
-                                                    natoms, P, status, status + 1);
+        int sms = 0;
+        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e == cudaSuccess)
+            e = launch_neighbors(sdev, sid, xw, xfc, xloc, cell_of, cell_start, cell_atoms, natoms, stencil_cells(s), 4, sms,
+                                 P, status, status + 1, st);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return NNAP_ERR_CUDA;
+        }
     }
     e = cudaGetLastError();
     if (e != cudaSuccess) return NNAP_ERR_CUDA;

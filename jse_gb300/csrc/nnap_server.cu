@@ -366,9 +366,11 @@ void submit_impl(nnap_server* s, int nslots, const int* ids, const double* const
         k_cell_order<<<(nb_atoms + 255) / 256, 256, 0, st>>>(h->cell_atoms.p, nb_atoms, h->xf.p, h->xlo.p, h->xfc.p,
                                                              h->xloc.p);
         const int nw = h->tune.nb_warps;
-        k_neighbors<<<(nb_atoms + nw - 1) / nw, 32 * nw, 0, st>>>(
-            s->sdev_build.p, sid, h->xw.p, h->xf.p, h->xlo.p, h->xfc.p, h->xloc.p, h->cell_of.p, h->cell_start.p,
-            h->cell_atoms.p, nb_atoms, pair_bufs(h), h->status.p, h->status.p + 1);
+        int max_off = 0;
+        for (auto& d : gsd) max_off = std::max(max_off, stencil_cells(d));
+        CK(launch_neighbors(s->sdev_build.p, sid, h->xw.p, h->xfc.p, h->xloc.p, h->cell_of.p, h->cell_start.p,
+                            h->cell_atoms.p, nb_atoms, max_off, nw, h->sm_count, pair_bufs(h), h->status.p,
+                            h->status.p + 1, st));
         k_verlet_store<<<(unsigned)(((size_t)nb_atoms * 32 + 127) / 128), 128, 0, st>>>(s->dslots.p, sid,
                                                                                        pair_bufs(h), nb_atoms,
                                                                                        s->kw.p);

@@ -3,6 +3,9 @@
 Backward descriptors: 32 lanes per atom below 4096 atoms and 16 from there (where two atoms' G
 fits), one- and several-species fuse matrices, more than three species (the sparse fuse
 tables), rows of fewer entries than a lane group, of whole groups and of one more.
+Neighbour rows: the chunk of atoms per warp (1, 2, 4 or 8 by the atom count), cells of the
+cutoff's width and of half of it, thin boxes with more stencil cells than are held at a time,
+batches that mix them.  Sets are compared exactly.
 
 Tolerances: a pair gradient is a sum of 2 N1 (lmax+1)^2, about a thousand, products of 24-bit
 numbers (2^-24 sqrt(1000) = 2e-6 of its terms) whose terms cancel to about a tenth: 2e-5 of the
@@ -51,3 +54,46 @@ FULL = {"type": "spherical_chebyshev", "nmax": 3, "lmax": 2, "rcut": 5.0, "wtype
 def test_backward_lanes(basis, T, n, density):
     s = W.random_liquid(n, density, [1.0 / T] * T, 1.9, n, tilt=0.1)
     _check(_model(basis, T), s)
+
+
+def _keys(off, j, img):
+    i = np.repeat(np.arange(len(off) - 1), np.diff(off))
+    img = np.asarray(img).reshape(-1, 3)
+    return np.unique(np.stack([i, j, img[:, 0], img[:, 1], img[:, 2]], 1), axis=0), len(j)
+
+
+def _same_rows(p, s, rcut):
+    off, j, img = p.neighborList(s)
+    nl = ON.neighbors(ON.wrap(s.x, s.box_kind, s.box), s.box_kind, s.box, rcut)
+    a, na = _keys(off, j, img)
+    b, nb = _keys(nl.offsets, nl.j, nl.img)
+    assert na == nb == len(a) and np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("rcut,n,tilt", [
+    (5.0, 1, None), (5.0, 9, 0.1), (5.0, 4863, None), (5.0, 14593, 0.1), (5.0, 29187, None), (5.0, 58370, 0.1),
+    (8.0, 3, 0.1), (8.0, 611, None), (8.0, 14593, 0.1), (8.0, 29190, None)])
+def test_neighbor_chunks(rcut, n, tilt):
+    from jse_gb300.nnap import NNAP
+    model = W.write_model(["A", "B"], {"type": "chebyshev", "nmax": 3, "rcut": rcut}, [4], 1)
+    s = W.random_liquid(n, 0.06, [0.5, 0.5], 1.9, n + 1, tilt=tilt)
+    with NNAP(model) as p:
+        _same_rows(p, s, rcut)
+
+
+def test_neighbor_thin_boxes():
+    from jse_gb300.nnap import NNAP
+    model = W.write_model(["A"], {"type": "chebyshev", "nmax": 3, "rcut": 6.0}, [4], 1)
+    rng = np.random.default_rng(4)
+    boxes = [np.diag([70.0, 2.3, 2.9]), np.diag([30.0, 5.0, 4.0]), np.diag([40.0, 33.0, 31.0])]
+    structures = []
+    for b in boxes:
+        n = max(1, int(0.05 * np.linalg.det(b)))
+        structures.append(W.Structure(rng.random((n, 3)) @ b, np.ones(n, dtype=np.int32), b, 0))
+    with NNAP(model) as p:
+        for s in structures:
+            _same_rows(p, s, 6.0)
+        both = p.calEnergyForceVirialsBatch(structures)
+        for s, o in zip(structures, both):
+            r = p.calEnergyForceVirials(s)
+            assert np.array_equal(r["forces"], o["forces"]) and np.array_equal(r["energies"], o["energies"])
