@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(32 * kDescMaxWarps) k_radial_fwd(DescArgs a) {
         float rcp = rc, ircp = irc;
         if (!pair_cut<RB>(a, tc, tn, r, rcp, ircp)) continue;
         float T[N1], sv[NP];
-        const float fc = radial_f<RB, N1>(r, ircp, T);
+        const float fc = radial_f<RB, N1>(r, rcp, ircp, T);
         fuse_apply<NP, N1>(sW + (size_t)(tc * a.T + tn) * NP * Fuse<N1>::N1P, T, sv);
 #pragma unroll
         for (int p = 0; p < NP; ++p) acc[p] += fc * sv[p];
@@ -156,6 +156,23 @@ struct SphShape {
     static constexpr int BWD_WARP_FLOATS = K * NPS + 2 * K * 32;
 };
 
+// Power spectrum of one atom from A [NP][K] in shared memory, a thread per channel: its K reads
+// walk the row with the loop over l unrolled (rows of odd length: no bank conflicts).
+template <int L, int NP>
+__device__ __forceinline__ void power_rows(const float* A, int nl2, int sl, float* __restrict__ out, int t, int nt) {
+    constexpr int K = (L + 1) * (L + 1);
+    for (int p = t; p < NP; p += nt) {
+        const float* row = A + p * K;
+#pragma unroll
+        for (int l = 0; l <= L; ++l) {
+            float s = 0.f;
+#pragma unroll
+            for (int m = 0; m <= 2 * l; ++m) s = fmaf(row[l * l + m], row[l * l + m], s);
+            if (l < nl2) out[p * sl + l] = kPi4 / (float)(2 * l + 1) * s;
+        }
+    }
+}
+
 template <int L, int NP, int N1, int RB>
 __global__ void __launch_bounds__(32 * kDescMaxWarps) k_sph_fwd(DescArgs a) {
     pdl_enter();
@@ -198,7 +215,7 @@ __global__ void __launch_bounds__(32 * kDescMaxWarps) k_sph_fwd(DescArgs a) {
             if (r < rc && pair_cut<RB>(a, tc, tn, r, rcp, ircp)) {
                 valid = true;
                 float T[N1], sv[NP];
-                const float fc = radial_f<RB, N1>(r, ircp, T);
+                const float fc = radial_f<RB, N1>(r, rcp, ircp, T);
                 fuse_apply<NP, N1>(sW + (size_t)(tc * a.T + tn) * NP * Fuse<N1>::N1P, T, sv);
 #pragma unroll
                 for (int p = 0; p < NP; ++p) c[p] = fc * sv[p];
@@ -235,9 +252,9 @@ __global__ void __launch_bounds__(32 * kDescMaxWarps) k_sph_fwd(DescArgs a) {
         }
         __syncwarp();
     }
-    // A to global (backward input) and squared to shared memory for the power spectrum
+    // A to global (backward input) and to shared memory for the power spectrum
     float* Aout = a.A + (size_t)w * NP * S::K;
-    float* sA2 = sY;
+    float* sA = sY;
 #pragma unroll
     for (int col = 0; col < S::COLS; ++col) {
         const int lm = lane + 32 * col;
@@ -246,17 +263,11 @@ __global__ void __launch_bounds__(32 * kDescMaxWarps) k_sph_fwd(DescArgs a) {
             for (int p = 0; p < NP; ++p) {
                 const float v = (p & 1) ? acc[p >> 1][col].y : acc[p >> 1][col].x;
                 Aout[p * S::K + lm] = v;
-                sA2[p * S::K + lm] = v * v;
+                sA[p * S::K + lm] = v;
             }
     }
     __syncwarp();
-    float* out = a.fp + (size_t)(s0 + w) * a.fp_stride + a.fp_off;
-    for (int e = lane; e < NP * a.nl2; e += 32) {
-        const int p = e / a.nl2, l = e - p * a.nl2;
-        float s = 0.f;
-        for (int m = 0; m <= 2 * l; ++m) s += sA2[p * S::K + l * l + m];
-        out[p * a.sl + l] = kPi4 / (float)(2 * l + 1) * s;
-    }
+    power_rows<L, NP>(sA, a.nl2, a.sl, a.fp + (size_t)(s0 + w) * a.fp_stride + a.fp_off, lane, 32);
 }
 
 // Forward in the space of the radial functions, for at most kFwdTypes species and fuse
@@ -280,6 +291,8 @@ struct SphFNShape {
     static constexpr int WARP_FLOATS = ((EVAL > POST ? EVAL : POST) + 3) & ~3;
 };
 
+// 1M-atom glass (lmax 4) 2.51 -> 2.04 ms with the angle-free harmonics and the spectrum by a
+// thread per channel (1500 warp instructions per atom; the shared-memory path is 75 % busy).
 template <int L, int NP, int N1>
 __global__ void __launch_bounds__(32 * kDescMaxWarps) k_sph_fwd_n(DescArgs a) {
     pdl_enter();
@@ -323,12 +336,12 @@ __global__ void __launch_bounds__(32 * kDescMaxWarps) k_sph_fwd_n(DescArgs a) {
             if (r < rc) {
                 valid = true;
                 tn = __float_as_int(d.w) - 1;
-                const float u = r * irc, fc1 = 1.f - u * u, fc2 = fc1 * fc1, fc = fc2 * fc2;
+                const float u = over_rc(r, rc, irc), fc1 = 1.f - u * u, fc2 = fc1 * fc1, fc = fc2 * fc2;
                 cheby_f<N1>(1.f - 2.f * u, fT);
 #pragma unroll
                 for (int n = 0; n < N1; ++n) fT[n] *= fc;
-                const Angles an = angles_f(d.x, d.y, d.z, r);
-                sph_harm<L, false>(an, y, nullptr, 1);
+                const float ir = 1.f / r;
+                sph_cart<L, false>(d.x * ir, d.y * ir, d.z * ir, y);
             }
         }
         if (!valid)
@@ -370,14 +383,15 @@ __global__ void __launch_bounds__(32 * kDescMaxWarps) k_sph_fwd_n(DescArgs a) {
         }
         __syncwarp();
     }
-    // A from the accumulators and alpha; A to global memory, A^2 to shared memory
-    float* sA2 = base;
+    // A from the accumulators and alpha, to global memory and to shared memory
+    float* sA = base;
     float* Aout = a.A + (size_t)w * NP * S::K;
     const float* al = sAl + (size_t)tc * kFwdTypes * NP;
 #pragma unroll
     for (int col = 0; col < S::COLS; ++col) {
         const int lm = lane + 32 * col;
         if (lm < S::K) {
+            const float4 nlm = d_shN[lm];  // the factor that Y left out
 #pragma unroll
             for (int p = 0; p < NP; ++p) {
                 const int n = p % N1;  // a constant once the loop is unrolled
@@ -385,19 +399,14 @@ __global__ void __launch_bounds__(32 * kDescMaxWarps) k_sph_fwd_n(DescArgs a) {
 #pragma unroll
                 for (int t = 0; t < kFwdTypes; ++t)
                     v += al[t * NP + p] * ((n & 1) ? acc[t][n >> 1][col].y : acc[t][n >> 1][col].x);
+                v = fmaf(v, nlm.x, v * nlm.y);
                 Aout[p * S::K + lm] = v;
-                sA2[p * S::K + lm] = v * v;
+                sA[p * S::K + lm] = v;
             }
         }
     }
     __syncwarp();
-    float* out = a.fp + (size_t)(s0 + w) * a.fp_stride + a.fp_off;
-    for (int e = lane; e < NP * a.nl2; e += 32) {
-        const int p = e / a.nl2, l = e - p * a.nl2;
-        float s = 0.f;
-        for (int m = 0; m <= 2 * l; ++m) s += sA2[p * S::K + l * l + m];
-        out[p * a.sl + l] = kPi4 / (float)(2 * l + 1) * s;
-    }
+    power_rows<L, NP>(sA, a.nl2, a.sl, a.fp + (size_t)(s0 + w) * a.fp_stride + a.fp_off, lane, 32);
 }
 
 // Backward, one warp per atom slot, one neighbour per lane.  For each neighbour,
@@ -465,7 +474,7 @@ __global__ void __launch_bounds__(32 * kDescMaxWarps, 2) k_sph_bwd(DescArgs a) {
         const float* Wt = sW + (size_t)(tc * a.T + tn) * NP * Fuse<N1>::N1P;
         if (valid) {
             float T[N1], sv[NP];
-            const float fc = radial_f<RB, N1>(r, ircp, T);
+            const float fc = radial_f<RB, N1>(r, rcp, ircp, T);
             fuse_apply<NP, N1>(Wt, T, sv);
 #pragma unroll
             for (int p = 0; p < NP; ++p) c[p] = fc * sv[p];
@@ -688,10 +697,9 @@ __global__ void __launch_bounds__(32 * kBwdWarps, LPA == 32 ? 5 : 6) k_sph_bwd_n
             for (m = 1; t >= L - m + 1; ++m) t -= L - m + 1;
             l0 = l1 = m + t;
         }
-        const float n0 = c_shN[tri(l0, m)], n1 = l1 <= L ? c_shN[tri(l1 <= L ? l1 : 0, m)] : 0.f;
-        sN[s] = make_float2(n0, n1);
-        sCo[s] = make_float2(l0 < a.nl2 ? n0 * (2.f * kPi4 / (float)(2 * l0 + 1)) : 0.f,
-                             l1 < a.nl2 ? n1 * (2.f * kPi4 / (float)(2 * l1 + 1)) : 0.f);
+        const float4 n0 = d_shN[l0 * l0 + l0 + m], n1 = d_shN[l1 <= L ? l1 * l1 + l1 + m : 0];
+        sN[s] = make_float2(n0.x, l1 <= L ? n1.x : 0.f);
+        sCo[s] = make_float2(l0 < a.nl2 ? n0.z : 0.f, l1 <= L && l1 < a.nl2 ? n1.z : 0.f);
     }
     __syncthreads();
     const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane / LPA, sub = lane % LPA;
@@ -818,7 +826,7 @@ __global__ void __launch_bounds__(32 * kBwdWarps, LPA == 32 ? 5 : 6) k_sph_bwd_n
         }
         const int tn = valid ? __float_as_int(d.w) - 1 : 0;
         const float ir = 1.f / r, x = d.x * ir, y = d.y * ir, z = d.z * ir;
-        const float u = r * irc, tx = 1.f - 2.f * u;
+        const float u = over_rc(r, rc, irc), tx = 1.f - 2.f * u;
         float Tn[N1];
         cheby_f<N1>(tx, Tn);
         float2 T2[N1], v2[N1];
@@ -852,7 +860,6 @@ __global__ void __launch_bounds__(32 * kBwdWarps, LPA == 32 ? 5 : 6) k_sph_bwd_n
             if (valid) {
                 // radial part: -(1/r) d/dr of fc and of T_n (n U_{n-1} 2 / (r rc))
                 const float fc1 = 1.f - u * u, fc2 = fc1 * fc1, fc = fc2 * fc2;
-                const float fcg = 8.f * fc1 * fc2 * irc * irc;
                 float dfc = v2[0].x + v2[0].y, drn = 0.f, um1 = 1.f, um2 = 0.f;
 #pragma unroll
                 for (int n = 1; n < N1; ++n) {
@@ -863,7 +870,7 @@ __global__ void __launch_bounds__(32 * kBwdWarps, LPA == 32 ? 5 : 6) k_sph_bwd_n
                     um2 = um1;
                     um1 = un;
                 }
-                const float gr = dfc * fcg + fc * (drn * (2.f * ir * irc));
+                const float gr = over_rc(over_rc(8.f * fc1 * fc2 * dfc, rc, irc) + fc * (drn * (2.f * ir)), rc, irc);
                 // a neighbour on the z axis has no phi terms (basis_SphericalUtil.hpp:160-181):
                 // phi = 0 there, so the y component of the angular part is dropped
                 if (fmaxf(fabsf(d.x), fabsf(d.y)) < 8.f * 1.17549435e-38f) gy = 0.f;
@@ -1204,7 +1211,7 @@ cudaError_t launch_sph(const DescArgs& a, bool fwd, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     if constexpr (RB == kRbNNAP) {   // the radial-space kernels are written for the NNAP radial functions
         if (!fwd && a.nz_p && a.nz_w && N1 <= NP) return launch_sph_bwd_n<L, NP, N1>(a, st);
-        if (fwd && a.fwd_alpha && N1 < NP && a.T <= kFwdTypes) {
+        if (fwd && a.fwd_alpha && N1 <= NP && a.T <= kFwdTypes) {
             if constexpr (SphTcShape<L, NP>::fits)
                 if (a.tc_sms > 0) return launch_sph_fwd_tc<L, NP, N1>(a, st);
             return launch_sph_fwd_n<L, NP, N1>(a, st);

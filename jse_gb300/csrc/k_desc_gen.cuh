@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps) k_radial_fwd_g(DescArgs a, int
                 float rcp = rc, ircp = irc;
                 if (r < rc && pair_cut_g<RB>(a, tc, t, r, rcp, ircp)) {
                     tn = t;
-                    const float fc = radial_f<RB, kMaxN1>(r, ircp, R);
+                    const float fc = radial_f<RB, kMaxN1>(r, rcp, ircp, R);
 #pragma unroll
                     for (int n = 0; n < kMaxN1; ++n) R[n] *= fc;
                 }
@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps) k_sph_fwd_g(DescArgs a, int NP
             if (r < rc && pair_cut_g<RB>(a, tc, tn, r, rcp, ircp)) {
                 valid = true;
                 float R[kMaxN1];
-                const float fc = radial_f<RB, kMaxN1>(r, ircp, R);
+                const float fc = radial_f<RB, kMaxN1>(r, rcp, ircp, R);
                 channel_row(a.W + ((size_t)tc * a.T + tn) * NP * N1, NP, NP8, N1, fc, R, cr);
                 sph_harm<L, false>(angles_f(d.x, d.y, d.z, r), y, nullptr, 1);
             }
@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps) k_sph_bwd_g(DescArgs a, int NP
         const float* Wt = a.W + ((size_t)tc * a.T + tn) * NP * N1;
         if (valid) {
             float R[kMaxN1];
-            const float fc = radial_f<RB, kMaxN1>(r, ircp, R);
+            const float fc = radial_f<RB, kMaxN1>(r, rcp, ircp, R);
             channel_row(Wt, NP, NP8, N1, fc, R, cr);
             sph_harm<L, true>(angles_f(d.x, d.y, d.z, r), y, yt, 1);
         } else {

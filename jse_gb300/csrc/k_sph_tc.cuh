@@ -11,7 +11,7 @@
 //
 // Precision.  Each FP32 operand x is split into FP16 hi = fp16(x) and lo = fp16(x - hi), and
 // each product is formed as hi*hi + lo*hi + hi*lo: about 22 significant bits per operand
-// where lo is a normal FP16 number (|x| >= 2^-3) and an absolute error below 2^-25
+// where lo is a normal FP16 number (|x| >= 2^-3) and an absolute error below 2^-25 (of 32 c)
 // otherwise, well inside FP32 descriptor accuracy.  The operands are bounded (|Y_lm| <= 1.5
 // for l <= 12, |fc T_n| <= 1), and the host uses this kernel only when every |alpha| is at
 // most kTcAlphaMax, so hi never overflows FP16.
@@ -25,7 +25,7 @@
 // atom's 32 TMEM columns and commits them to the warp's mbarrier.  After the round's last
 // MMAs all 4 warps read the 4 tiles back: an M = 64 tile keeps rows 16q..16q+15 in TMEM
 // lanes 32q..32q+15, which warp q reads.  They write A and form the power spectrum from
-// A^2 in shared memory (the operand buffers, free once the MMAs are done).  Every wait on
+// A in shared memory (the operand buffers, free once the MMAs are done).  Every wait on
 // an mbarrier is bounded; a wait that gives up raises ERRBIT_TIMEOUT.
 #pragma once
 
@@ -37,26 +37,31 @@ namespace nnapgb {
 namespace {
 
 constexpr int kFwdTcWarps = 4;
+// c is split times this (kTcAlphaMax times it is below FP16's largest number), so that the lo
+// part of a neighbour near the cutoff, where fc is small, stays clear of FP16's smallest steps.
+constexpr float kTcScale = 32.f;
 
 template <int L, int NP>
 struct SphTcShape {
     static constexpr int KM = (L + 1) * (L + 1);   // tile rows in use
     static constexpr int NPN = (NP + 7) & ~7;       // MMA N
     static constexpr int NCA = (KM + 7) / 8;        // 8-row groups of Y a neighbour writes
+    static constexpr int NPH = NPN / 2 <= 4 ? 4 : NPN / 2 <= 8 ? 8 : 16;  // columns a lane reads back
     static constexpr int NCB = NPN / 8;             // 8-column groups of c a neighbour writes
     static constexpr int ABYTES = 64 * 16 * 2;      // one FP16 image of a chunk's Y^T
     static constexpr int BBYTES = 16 * NPN * 2;     // one FP16 image of a chunk's C
     static constexpr int CHUNK = 2 * ABYTES + 2 * BBYTES;
     static constexpr int WARP_BYTES = 2 * CHUNK;
-    static constexpr int AL_BYTES = (kFwdTypes * kFwdTypes * NP * 4 + 127) & ~127;
+    static constexpr int AL_BYTES = (kFwdTypes * kFwdTypes * NPN * 4 + 127) & ~127;
     static constexpr int A2_BYTES = kFwdTcWarps * NP * KM * 4;
     static constexpr int OPS = kFwdTcWarps * WARP_BYTES > A2_BYTES ? kFwdTcWarps * WARP_BYTES : A2_BYTES;
     // at least 46 KB, so that at most four CTAs (4 x 128 TMEM columns) share an SM
     static constexpr int SMEM = AL_BYTES + OPS > 47104 ? AL_BYTES + OPS : 47104;
-    // lmax 6 or 7: the tile's 64 rows are mostly in use.  Below that the FP32-pipe kernel,
-    // whose work scales with (L+1)^2, is faster (lmax 4, 131k-atom glass: 0.34 against
-    // 0.41 ms; lmax 6, 1024-structure batch: 2.41 against 2.08 ms on the tensor cores)
-    static constexpr bool fits = KM >= 49 && KM <= 64 && NPN <= 32;
+    // lmax 6 or 7, where the tile's 64 rows are mostly in use, and 16 or more channels.  Each MMA
+    // truncates its FP32 accumulation, so descriptors are within 9e-7 of 64 bits where the FP32
+    // pipe's are within 3e-7: smaller shapes, which gain less, stay there (lmax 4 with two atoms
+    // per tile: 1.65 against 2.05 ms on the 1M-atom glass)
+    static constexpr bool fits = KM >= 49 && KM <= 64 && NP >= 16 && NPN <= 32;
 };
 
 __device__ __forceinline__ uint64_t tc_sdesc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
@@ -75,7 +80,8 @@ __device__ __forceinline__ void split_f16x8(const float* v, uint4& hi, uint4& lo
     for (int q = 0; q < 4; ++q) {
         const __half2 hh = __floats2half2_rn(v[2 * q], v[2 * q + 1]);
         const float2 hf = __half22float2(hh);
-        const __half2 ll = __floats2half2_rn(v[2 * q] - hf.x, v[2 * q + 1] - hf.y);
+        const float2 lf = __ffma2_rn(hf, make_float2(-1.f, -1.f), make_float2(v[2 * q], v[2 * q + 1]));
+        const __half2 ll = __floats2half2_rn(lf.x, lf.y);
         h[q] = *reinterpret_cast<const uint32_t*>(&hh);
         l[q] = *reinterpret_cast<const uint32_t*>(&ll);
     }
@@ -83,21 +89,47 @@ __device__ __forceinline__ void split_f16x8(const float* v, uint4& hi, uint4& lo
     lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
-// 32 TMEM columns of this warp's lane quarter, waited for in the same statement.
-__device__ __forceinline__ void tmem_ld32_wait(uint32_t taddr, float* v) {
-    uint32_t r[32];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
+// Bound: instruction issue (1716 warp instructions per atom of 54 neighbours, 53 % of the slots;
+// the operand splits and stores are a third).  Angle-free harmonics, a read-back by both halves
+// of each warp, the spectrum by a thread per channel and the next atom's loads ahead of their
+// use: 1024-structure batch 2.00 -> 1.32 ms, 32000-atom liquid 139 -> 97 us.
+
+// TMEM lanes 0..15 of this warp's quarter, both halves of the warp reading: lanes 0..15 the
+// columns from taddr, lanes 16..31 those from taddr + H (the next 4, 8 or 16 columns of each),
+// waited for in the same statement.
+template <int H>
+__device__ __forceinline__ void tmem_ld_halves_wait(uint32_t taddr, float* v) {
+    if constexpr (H <= 4) {
+        uint32_t r[4];
+        asm volatile("tcgen05.ld.sync.aligned.16x32bx2.x4.b32 {%0,%1,%2,%3}, [%4], %5;\n\t"
+                     "tcgen05.wait::ld.sync.aligned;"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(taddr), "n"(H)
+                     : "memory");
 #pragma unroll
-    for (int q = 0; q < 32; ++q) v[q] = __uint_as_float(r[q]);
+        for (int q = 0; q < 4; ++q) v[q] = __uint_as_float(r[q]);
+    } else if constexpr (H <= 8) {
+        uint32_t r[8];
+        asm volatile("tcgen05.ld.sync.aligned.16x32bx2.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8], %9;\n\t"
+                     "tcgen05.wait::ld.sync.aligned;"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                     : "r"(taddr), "n"(H)
+                     : "memory");
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = __uint_as_float(r[q]);
+    } else {
+        uint32_t r[16];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.16x32bx2.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16], "
+            "%17;\n\t"
+            "tcgen05.wait::ld.sync.aligned;"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+              "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+            : "r"(taddr), "n"(H)
+            : "memory");
+#pragma unroll
+        for (int q = 0; q < 16; ++q) v[q] = __uint_as_float(r[q]);
+    }
 }
 
 template <int L, int NP, int N1>
@@ -110,11 +142,14 @@ __global__ void __launch_bounds__(32 * kFwdTcWarps, 4) k_sph_fwd_tc(DescArgs a) 
     __shared__ uint32_t s_tmem;
     __shared__ int s_cnt[kFwdTcWarps];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int ntab = a.T * kFwdTypes * NP;
+    const int ntab = a.T * kFwdTypes * NPN;  // alpha[tc][tn][p], rows padded to NPN
     float* sAl = reinterpret_cast<float*>(smem);
     uint8_t* ops = smem + S::AL_BYTES;
-    float* sA2 = reinterpret_cast<float*>(ops);  // [warp][NP][KM] once a round's MMAs are done
-    for (int q = tid; q < ntab; q += blockDim.x) sAl[q] = a.fwd_alpha[q];
+    float* sA = reinterpret_cast<float*>(ops);  // [warp][NP][KM] once a round's MMAs are done
+    for (int q = tid; q < ntab; q += blockDim.x) {
+        const int row = q / NPN, p = q - row * NPN;
+        sAl[q] = p < NP ? kTcScale * a.fwd_alpha[row * NP + p] : 0.f;
+    }
     if (tid == 0) {
         for (int q = 0; q < kFwdTcWarps; ++q)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc::smem_u32(&mbar[q])) : "memory");
@@ -147,46 +182,64 @@ __global__ void __launch_bounds__(32 * kFwdTcWarps, 4) k_sph_fwd_tc(DescArgs a) 
     const int aoff = (kk >> 3) * 1024 + (kk & 7) * 16;
     const int boff = (kk >> 3) * (NPN / 8) * 128 + (kk & 7) * 16;
 
-    for (int r0 = blockIdx.x * kFwdTcWarps; r0 < nslot; r0 += gridDim.x * kFwdTcWarps) {
-        const int slot = r0 + warp;
-        int at = 0, tc = 0, cnt = 0;
-        if (slot < nslot) {
-            at = a.perm[s0 + slot];
-            tc = a.type[at] - 1;
-            cnt = min(a.P.count[at], M);
-        }
+    // the first neighbours of the next round's atom are loaded while this round computes
+    int at = 0, tc = 0, cnt = 0;
+    float4 d0 = make_float4(0.f, 0.f, 1.f, __int_as_float(1));
+    const int rstep = gridDim.x * kFwdTcWarps;
+    int r0 = blockIdx.x * kFwdTcWarps;
+    if (r0 + warp < nslot) {
+        at = a.perm[s0 + r0 + warp];
+        tc = a.type[at] - 1;
+        cnt = min(a.P.count[at], M);
+        if (lane < cnt) d0 = a.P.dx[(size_t)at * M + lane];
+    }
+    for (; r0 < nslot; r0 += rstep) {
         if (lane == 0) s_cnt[warp] = cnt;
-        const float* al = sAl + tc * kFwdTypes * NP;
+        int at_n = -1, tc_n = 0, cnt_n = 0;
+        float4 dn = make_float4(0.f, 0.f, 1.f, __int_as_float(1));
+        if (r0 + rstep + warp < nslot) at_n = a.perm[s0 + r0 + rstep + warp];
+        const float* al = sAl + tc * kFwdTypes * NPN;
         for (int b0 = 0; b0 < cnt; b0 += 32) {
             const int k = b0 + lane;
+            const float4 dl = d0;
+            if (k + 32 < cnt) d0 = a.P.dx[(size_t)at * M + k + 32];  // the next step's
             float y[KM];
             float c[NPN];
-#pragma unroll
-            for (int p = 0; p < NPN; ++p) c[p] = 0.f;
+            // a lane without a neighbour takes c = 0 and the harmonics of the z axis
+            float4 d = make_float4(0.f, 0.f, 1.f, __int_as_float(1));
+            float r = 1.f;
             bool valid = false;
             if (k < cnt) {
-                const float4 d = a.P.dx[(size_t)at * M + k];
-                const float r = sqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
-                if (r < rc) {
-                    valid = true;
-                    const int tn = __float_as_int(d.w) - 1;
-                    const float u = r * irc, fc1 = 1.f - u * u, fc2 = fc1 * fc1, fc = fc2 * fc2;
-                    float fT[N1];
-                    cheby_f<N1>(1.f - 2.f * u, fT);
-#pragma unroll
-                    for (int p = 0; p < NP; ++p) c[p] = al[tn * NP + p] * (fc * fT[p % N1]);
-                    const Angles an = angles_f(d.x, d.y, d.z, r);
-                    sph_harm<L, false>(an, y, nullptr, 1);
-                }
+                d = dl;
+                r = sqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
+                valid = r < rc;
             }
-            if (!valid) {
+            {
+                const int tn = __float_as_int(d.w) - 1;
+                const float u = over_rc(r, rc, irc), fc1 = 1.f - u * u, fc2 = fc1 * fc1, fc = valid ? fc2 * fc2 : 0.f;
+                float fT[N1];
+                cheby_f<N1>(1.f - 2.f * u, fT);
+                const float4* a4 = reinterpret_cast<const float4*>(al + tn * NPN);
 #pragma unroll
-                for (int q = 0; q < KM; ++q) y[q] = 0.f;
+                for (int q = 0; q < NPN / 4; ++q) {
+                    const float4 v = a4[q];
+                    const float w4[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int p = 4 * q + e;
+                        c[p] = p < NP ? w4[e] * (fc * fT[p % N1]) : 0.f;
+                    }
+                }
+                const float ir = 1.f / r;
+                sph_cart<L, true>(d.x * ir, d.y * ir, d.z * ir, y);
             }
             // the warp's previous MMAs read these chunks
             if (b0 > 0) {
                 ok = tc::mbar_wait(mb, phase) && ok;
                 phase ^= 1;
+            } else if (at_n >= 0) {
+                tc_n = a.type[at_n] - 1;
+                cnt_n = min(a.P.count[at_n], M);
             }
 #pragma unroll
             for (int g = 0; g < S::NCA; ++g) {
@@ -223,6 +276,13 @@ __global__ void __launch_bounds__(32 * kFwdTcWarps, 4) k_sph_fwd_tc(DescArgs a) 
             }
             __syncwarp();
         }
+        if (at_n >= 0) {
+            if (cnt == 0) {
+                tc_n = a.type[at_n] - 1;
+                cnt_n = min(a.P.count[at_n], M);
+            }
+            if (lane < cnt_n) dn = a.P.dx[(size_t)at_n * M + lane];
+        }
         if (cnt > 0) {
             ok = tc::mbar_wait(mb, phase) && ok;
             phase ^= 1;
@@ -230,37 +290,48 @@ __global__ void __launch_bounds__(32 * kFwdTcWarps, 4) k_sph_fwd_tc(DescArgs a) 
         tc::fence_before();
         __syncthreads();
         tc::fence_after();
-        // the 4 tiles: warp q holds rows lm = 16q + lane (lanes 0..15)
+        // the 4 tiles: warp q reads rows lm = 16q + (lane & 15), lanes 0..15 the first half of the
+        // columns and lanes 16..31 the second
         for (int w4 = 0; w4 < kFwdTcWarps; ++w4) {
             const int sl = r0 + w4;
             if (sl >= nslot) break;
-            float v[32];
-            tmem_ld32_wait(tbase + ((uint32_t)(32 * warp) << 16) + 32u * w4, v);
-            const int lm = 16 * warp + lane;
-            if (lane < 16 && lm < KM) {
+            float v[S::NPH];
+            tmem_ld_halves_wait<NPN / 2>(tbase + ((uint32_t)(32 * warp) << 16) + 32u * w4, v);
+            const int lm = 16 * warp + (lane & 15), p0 = (lane >> 4) * (NPN / 2);
+            if (lm < KM) {
                 const bool any = s_cnt[w4] > 0;
-                float* Aout = a.A + (size_t)sl * NP * KM;
-                float* a2 = sA2 + w4 * NP * KM;
+                float* Aout = a.A + (size_t)sl * NP * KM + p0 * KM + lm;
+                float* sa = sA + w4 * NP * KM + p0 * KM + lm;
 #pragma unroll
-                for (int p = 0; p < NP; ++p) {
-                    const float x = any ? v[p] : 0.f;
-                    Aout[p * KM + lm] = x;
-                    a2[p * KM + lm] = x * x;
+                for (int p = 0; p < NPN / 2; ++p) {
+                    if (p0 + p < NP) {
+                        const float x = any ? v[p] * (1.f / kTcScale) : 0.f;
+                        Aout[p * KM] = x;
+                        sa[p * KM] = x;
+                    }
                 }
             }
         }
         __syncthreads();
-        const int nout = NP * a.nl2;
-        for (int e = tid; e < kFwdTcWarps * nout; e += blockDim.x) {
-            const int w4 = e / nout, rr = e - w4 * nout;
+        // power spectrum: a thread per (atom, channel)
+        for (int e = tid; e < kFwdTcWarps * NP; e += blockDim.x) {
+            const int w4 = e / NP, p = e - w4 * NP;
             const int sl = r0 + w4;
             if (sl >= nslot) continue;
-            const int p = rr / a.nl2, l = rr - p * a.nl2;
-            const float* a2 = sA2 + w4 * NP * KM + p * KM + l * l;
-            float s = 0.f;
-            for (int m = 0; m <= 2 * l; ++m) s += a2[m];
-            a.fp[(size_t)(s0 + sl) * a.fp_stride + a.fp_off + p * a.sl + l] = kPi4 / (float)(2 * l + 1) * s;
+            const float* row = sA + e * KM;
+            float* out = a.fp + (size_t)(s0 + sl) * a.fp_stride + a.fp_off + p * a.sl;
+#pragma unroll
+            for (int l = 0; l <= L; ++l) {
+                float s = 0.f;
+#pragma unroll
+                for (int m = 0; m <= 2 * l; ++m) s = fmaf(row[l * l + m], row[l * l + m], s);
+                if (l < a.nl2) out[l] = kPi4 / (float)(2 * l + 1) * s;
+            }
         }
+        at = at_n;
+        tc = tc_n;
+        cnt = cnt_n;
+        d0 = dn;
         tc::fence_before();
         __syncthreads();
         tc::fence_after();

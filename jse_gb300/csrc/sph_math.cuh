@@ -18,6 +18,10 @@ __constant__ float c_shA[91], c_shB[91], c_dup[91], c_ddn[91];
 __constant__ float c_diag[13], c_sub[13];
 // Factors of the monic harmonics (below): Y_{l,+-m} = c_shN[tri(l,m)] Q_lm(z) {Re, Im}(x + iy)^m.
 __constant__ float c_shN[91];
+// By lm = l^2 + l + m: N_lm as hi + lo (sums scaled by it carry no rounding of the factor, which
+// would be the same for every neighbour and atom and so add up in a total virial) and
+// N_lm 2 4pi/(2l+1).
+__device__ float4 d_shN[169];
 
 // Recursion coefficients of the normalised associated Legendre functions for l <= 12.
 cudaError_t upload_sh_tables() {
@@ -35,13 +39,17 @@ cudaError_t upload_sh_tables() {
     // sqrt2 (m > 0) (-1)^m sqrt((2l+1)/(4 pi) (l-m)!/(l+m)!) times the leading coefficient
     // (2l-1)!!/(l-m)! of d^m P_l / dz^m
     float nm[91] = {0};
+    float4 nlm[169];
     for (int l = 0; l <= 12; ++l)
         for (int m = 0; m <= l; ++m) {
             double f = (2.0 * l + 1.0) / 12.566370614359172, c = 1.0;
             for (int k = l - m + 1; k <= l + m; ++k) f /= k;
             for (int k = 1; k <= l; ++k) c *= 2.0 * k - 1.0;
             for (int k = 1; k <= l - m; ++k) c /= k;
-            nm[l * (l + 1) / 2 + m] = (float)((m & 1 ? -1.0 : 1.0) * sqrt(m ? 2.0 * f : f) * c);
+            const double v = (m & 1 ? -1.0 : 1.0) * sqrt(m ? 2.0 * f : f) * c;
+            nm[l * (l + 1) / 2 + m] = (float)v;
+            nlm[l * l + l + m] = nlm[l * l + l - m] = 
+                make_float4((float)v, (float)(v - (double)(float)v), (float)(v * 25.132741228718345 / (2.0 * l + 1.0)), 0.f);
         }
     for (int m = 0; m <= 12; ++m) {
         dg[m] = m ? (float)sqrt(1.0 + 0.5 / m) : 0.f;
@@ -54,6 +62,7 @@ cudaError_t upload_sh_tables() {
     if ((e = cudaMemcpyToSymbol(c_ddn, dn, sizeof(dn))) != cudaSuccess) return e;
     if ((e = cudaMemcpyToSymbol(c_diag, dg, sizeof(dg))) != cudaSuccess) return e;
     if ((e = cudaMemcpyToSymbol(c_shN, nm, sizeof(nm))) != cudaSuccess) return e;
+    if ((e = cudaMemcpyToSymbol(d_shN, nlm, sizeof(nlm))) != cudaSuccess) return e;
     return cudaMemcpyToSymbol(c_sub, sb, sizeof(sb));
 }
 
@@ -82,6 +91,12 @@ __device__ __forceinline__ void cheby_grad_f(float x, float mul, float* G) {
     }
 }
 
+// r / rc through irc = 1 / rc (rounded) and its residual (1 - rc irc) / rc: the rounding of irc
+// alone would scale every distance alike (lmax 4 glass, cutoff 5.5: 4e-6 of the total virial).
+__device__ __forceinline__ float over_rc(float r, float rc, float irc) {
+    return fmaf(r, irc, r * (fmaf(-rc, irc, 1.f) * irc));
+}
+
 // Radial functions of the two bases the p-space descriptor kernels serve (template
 // parameter RB); a neighbour's channel value is c_p = fc sum_n W[p][n] R_n.
 //   kRbNNAP (nnap_util.hpp:226-271):            u = r/rc, fc = (1 - u^2)^4, R_n = T_n(1 - 2u)
@@ -90,8 +105,8 @@ __device__ __forceinline__ void cheby_grad_f(float x, float mul, float* G) {
 // radial_f returns fc and fills R; radial_g also fills RG_n = -(1/r) dR_n/dr and sets
 // fcg = -(1/r) dfc/dr.
 template <int RB, int N1>
-__device__ __forceinline__ float radial_f(float r, float irc, float* R) {
-    const float u = r * irc;
+__device__ __forceinline__ float radial_f(float r, float rc, float irc, float* R) {
+    const float u = RB == kRbNEP ? r * irc : over_rc(r, rc, irc);
     if (RB == kRbNEP) {
         cheby_f<N1>(2.f * (u - 1.f) * (u - 1.f) - 1.f, R);
 #pragma unroll
@@ -105,7 +120,7 @@ __device__ __forceinline__ float radial_f(float r, float irc, float* R) {
 
 template <int RB, int N1>
 __device__ __forceinline__ float radial_g(float r, float rc, float irc, float* R, float* RG, float* fcg) {
-    const float u = r * irc;
+    const float u = RB == kRbNEP ? r * irc : over_rc(r, rc, irc);
     if (RB == kRbNEP) {
         const float x = 2.f * (u - 1.f) * (u - 1.f) - 1.f;
         cheby_f<N1>(x, R);
@@ -159,6 +174,34 @@ __device__ __forceinline__ void monic_column(float z, float* q) {
     if (m + 1 <= L) q[m + 1] = z;
 #pragma unroll
     for (int l = m + 2; l <= L; ++l) q[l] = fmaf(z, q[l - 1], -leg_beta(l, m) * q[l - 2]);
+}
+
+// Y[lm] of a unit vector through the monic columns; without NORM, Y / N_lm (the caller scales its
+// sums by d_shN).
+template <int L, bool NORM>
+__device__ __forceinline__ void sph_cart(float x, float y, float z, float* Y) {
+    float cm = 1.f, sm = 0.f;
+#pragma unroll
+    for (int m = 0; m <= L; ++m) {
+        float q1 = 0.f, q2 = 0.f;  // Q_{l-1,m}, Q_{l-2,m}
+#pragma unroll
+        for (int l = m; l <= L; ++l) {
+            float q = l == m ? 1.f : l == m + 1 ? z : fmaf(z, q1, -leg_beta(l, m) * q2);
+            q2 = q1;
+            q1 = q;
+            if (NORM) q *= c_shN[tri(l, m)];
+            const int c0 = l * l + l;
+            if (m == 0) {
+                Y[c0] = q;
+            } else {
+                Y[c0 + m] = q * cm;
+                Y[c0 - m] = q * sm;
+            }
+        }
+        const float cn = fmaf(x, cm, -(y * sm)), sn = fmaf(x, sm, y * cm);
+        cm = cn;
+        sm = sn;
+    }
 }
 
 struct Angles {

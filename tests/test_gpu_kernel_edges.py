@@ -6,6 +6,9 @@ tables), rows of fewer entries than a lane group, of whole groups and of one mor
 Neighbour rows: the chunk of atoms per warp (1, 2, 4 or 8 by the atom count), cells of the
 cutoff's width and of half of it, thin boxes with more stencil cells than are held at a time,
 batches that mix them.  Sets are compared exactly.
+Forward descriptors on the tensor cores: rounds of four atoms with one to five atoms in them,
+atoms without a neighbour, rows of more than 64.  A coefficient is the sum of up to 15 MMAs that
+each truncate it (2^-23), squared: 4e-6 of a column's scale, tested at 1e-5.
 
 Tolerances: a pair gradient is a sum of 2 N1 (lmax+1)^2, about a thousand, products of 24-bit
 numbers (2^-24 sqrt(1000) = 2e-6 of its terms) whose terms cancel to about a tenth: 2e-5 of the
@@ -97,3 +100,17 @@ def test_neighbor_thin_boxes():
         for s, o in zip(structures, both):
             r = p.calEnergyForceVirials(s)
             assert np.array_equal(r["forces"], o["forces"]) and np.array_equal(r["energies"], o["energies"])
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp32"])
+@pytest.mark.parametrize("n,density", [(1, 0.001), (2, 0.003), (3, 0.06), (5, 0.012), (33, 0.06), (66, 0.083)])
+def test_forward_descriptors(precision, n, density):
+    from jse_gb300.nnap import NNAP
+    basis = {"type": "spherical_chebyshev", "nmax": 8, "lmax": 6, "rcut": 6.0}
+    model = W.write_model(["A", "B", "C"], basis, [8], 2)
+    s = W.random_liquid(n, density, [0.4, 0.4, 0.2], 1.8, n, tilt=0.1)
+    ref = ON.compute(OM.load(model), s.x, s.types, s.box_kind, s.box, want_fp=True)["fp"]
+    with NNAP(model, precision=precision) as p:
+        fp = p.calFp(s)
+    scale = np.abs(ref).max(0) + 1e-6
+    assert (np.abs(fp - ref) / scale).max() <= 1e-5
