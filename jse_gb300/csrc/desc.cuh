@@ -144,7 +144,8 @@ struct NetArgs {
 };
 
 // FP32 SIMT network (plain precision).
-cudaError_t launch_net_fp32(const NetArgs& a, cudaStream_t st);
+// count species (one launch); a[k].t names the species.
+cudaError_t launch_net_fp32(const NetArgs* a, int count, int sms, cudaStream_t st);
 // Whether the FP32 network of this shape fits in shared memory (at least one warp per CTA).
 bool net_fp32_fits(int D, int nlayer, const int* H);
 

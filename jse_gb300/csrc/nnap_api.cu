@@ -695,7 +695,7 @@ void enqueue_eval(nnap_handle* h, const Batch& B, const int* d_type, bool fp_onl
     descriptors(true);
     h->mark(2);
     if (!fp_only && n > 0) {
-        std::vector<NetArgs> args(T);
+        std::vector<NetArgs> args(T), plain;
         for (int t = 0; t < T; ++t) {
             const NetDev& nd = h->nets[t];
             NetArgs& a = args[t];
@@ -714,10 +714,11 @@ void enqueue_eval(nnap_handle* h, const Batch& B, const int* d_type, bool fp_onl
             a.e_atom = h->e_atom.p;
             a.gfp = h->gfp.p;
             a.act = nd.act;
-            if (!(h->net_tc && nd.tc.ready)) {
-                CK(launch_net_fp32(a, st));
-                ++h->launches;
-            }
+            if (!(h->net_tc && nd.tc.ready)) plain.push_back(a);
+        }
+        if (!plain.empty()) {
+            CK(launch_net_fp32(plain.data(), (int)plain.size(), h->sm_count, st));
+            ++h->launches;
         }
         if (h->net_tc) {
             // one launch per run of consecutive tensor-core species with the same network layout

@@ -6,6 +6,7 @@ tables), rows of fewer entries than a lane group, of whole groups and of one mor
 Neighbour rows: the chunk of atoms per warp (1, 2, 4 or 8 by the atom count), cells of the
 cutoff's width and of half of it, thin boxes with more stencil cells than are held at a time,
 batches that mix them.  Sets are compared exactly.
+FP32 network: see its test.
 Forward descriptors on the tensor cores: rounds of four atoms with one to five atoms in them,
 atoms without a neighbour, rows of more than 64.  A coefficient is the sum of up to 15 MMAs that
 each truncate it (2^-23), squared: 4e-6 of a column's scale, tested at 1e-5.
@@ -114,3 +115,21 @@ def test_forward_descriptors(precision, n, density):
         fp = p.calFp(s)
     scale = np.abs(ref).max(0) + 1e-6
     assert (np.abs(fp - ref) / scale).max() <= 1e-5
+
+
+@pytest.mark.parametrize("T,nmax,hidden,n", [
+    (1, 10, (32, 32), 5), (1, 10, (33,), 9), (2, 15, (31,), 40), (3, 20, (64, 7, 40), 1), (3, 20, (64, 7, 40), 17),
+    (3, 20, (300, 20), 33), (2, 15, (64, 64), 3700)])
+def test_network_slices(T, nmax, hidden, n):
+    """The FP32 network by a warp, a CTA or without slices per eight atoms: layers of up to one, of
+    exactly one and of several slices, more units than a CTA's threads, the last group of atoms
+    short, a batch equal to its structures alone.  Sums of up to 300 products: 2^-24 sqrt(300) =
+    1e-6 of the terms."""
+    from jse_gb300.nnap import NNAP
+    model = _model({"type": "chebyshev", "nmax": nmax, "rcut": 5.0}, T, hidden)
+    s = W.random_liquid(n, 0.05, [1.0 / T] * T, 1.9, n)
+    _check(model, s)
+    small = W.random_liquid(13, 0.05, [1.0 / T] * T, 1.9, 2)
+    with NNAP(model) as p:
+        for a, b in zip(p.calEnergyForceVirialsBatch([small, s]), [p.calEnergyForceVirials(small), p.calEnergyForceVirials(s)]):
+            assert np.array_equal(a["energies"], b["energies"]) and np.array_equal(a["forces"], b["forces"])
