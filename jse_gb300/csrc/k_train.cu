@@ -472,7 +472,7 @@ __device__ __forceinline__ void mv_fwd(const float* __restrict__ WT, const float
             za[q] = (bias && ha) ? bias[oa] : 0.f;
             zb[q] = (bias && hb) ? bias[ob] : 0.f;
         }
-#pragma unroll 4
+#pragma unroll 8
         for (int i = 0; i < in; ++i) {
             const float wa = ha ? WT[(size_t)i * H + oa] : 0.f;
             const float wb = hb ? WT[(size_t)i * H + ob] : 0.f;
@@ -503,7 +503,7 @@ __device__ __forceinline__ void mv_bwd(const float* __restrict__ W, int in, int 
 #pragma unroll
             for (int q = 0; q < kTrainAtoms; ++q) g[r][q] = 0.f;
         }
-#pragma unroll 2
+#pragma unroll 4
         for (int o = 0; o < H; ++o) {
             const float4 d0 = *reinterpret_cast<const float4*>(vin + o * kTrainAtoms);
             const float4 d1 = *reinterpret_cast<const float4*>(vin + o * kTrainAtoms + 4);
@@ -533,8 +533,15 @@ __device__ __forceinline__ void put_rec(float* rec, int V, int slot0, int na, in
 
 // One warp per 8 atom slots of one species.  Shared memory per warp (units x 8 atoms):
 // x, ux [D]; z_l, aH_l [H_l] per layer; two work buffers [Hmax].
-__global__ void __launch_bounds__(128) k_net_train(NetTrainArgs a, int warp_floats) {
+struct NetTrainMulti {
+    NetTrainArgs a[kMaxTypes];
+};
+
+// All species in one launch (blockIdx.y): the time of a small batch is the chain of weight loads
+// (2600 atoms, two species 50-32-32: 123 us as a launch each with half the loads in flight -> 62 us).
+__global__ void __launch_bounds__(128) k_net_train(const __grid_constant__ NetTrainMulti m, int warp_floats) {
     extern __shared__ float smem[];
+    const NetTrainArgs& a = m.a[blockIdx.y];
     const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int s0 = a.range[a.t], s1 = a.range[a.t + 1];
     const int slot0 = s0 + (blockIdx.x * (blockDim.x >> 5) + wl) * kTrainAtoms;
@@ -1008,12 +1015,29 @@ __global__ void __launch_bounds__(32 * kWgWarps) k_wgrad(WgradArgs g) {
     }
 }
 
-__global__ void k_wgrad_final(const float* __restrict__ partial, int G, int per, double* __restrict__ out) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= per) return;
+// A CTA per 8 entries, 32 rows of threads: row r adds partials r, r + 32, .. and the 32 sums are
+// added in order, in FP64.  Few entries per CTA spread the FP64 additions, whose pipe takes two
+// per cycle and SM, over more SMs.  2600 partials of 200 entries: one thread per entry through
+// all partials 320 us, 32 entries per CTA 45, 8 entries 25.
+constexpr int kFinalRows = 32, kFinalCols = 8;
+
+__global__ void __launch_bounds__(kFinalCols * kFinalRows) k_wgrad_final(const float* __restrict__ partial, int G, int per,
+                                                                         double* __restrict__ out) {
+    __shared__ double sums[kFinalRows][kFinalCols];
+    const int c = threadIdx.x % kFinalCols, r = threadIdx.x / kFinalCols, e = blockIdx.x * kFinalCols + c;
     double s = 0.0;
-    for (int w = 0; w < G; ++w) s += (double)partial[(size_t)w * per + e];
-    out[e] = s;
+    if (e < per) {
+#pragma unroll 8
+        for (int w = r; w < G; w += kFinalRows) s += (double)partial[(size_t)w * per + e];
+    }
+    sums[r][c] = s;
+    __syncthreads();
+    if (r == 0 && e < per) {
+        double t = 0.0;
+#pragma unroll
+        for (int q = 0; q < kFinalRows; ++q) t += sums[q][c];
+        out[e] = t;
+    }
 }
 
 // =========================================================================== launchers
@@ -1106,7 +1130,7 @@ cudaError_t launch_wgrad(int kind, int lmax, int np, int n1, const WgradArgs& a,
 
 cudaError_t launch_wgrad_final(const float* partial, int G, int per, double* out, cudaStream_t st) {
     if (per <= 0) return cudaSuccess;
-    k_wgrad_final<<<(per + 255) / 256, 256, 0, st>>>(partial, G, per, out);
+    k_wgrad_final<<<(per + kFinalCols - 1) / kFinalCols, kFinalCols * kFinalRows, 0, st>>>(partial, G, per, out);
     return cudaGetLastError();
 }
 
@@ -1126,15 +1150,22 @@ cudaError_t launch_jvp(int kind, int lmax, int np, int n1, const JvpArgs& a, cud
     return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_net_train(const NetTrainArgs& a, cudaStream_t st) {
-    const int n = a.nmax;
+cudaError_t launch_net_train(const NetTrainArgs* args, int count, cudaStream_t st) {
+    if (count <= 0 || count > kMaxTypes) return count ? cudaErrorInvalidValue : cudaSuccess;
+    const int n = args[0].nmax;
     if (n <= 0) return cudaSuccess;
-    int Hmax = a.D, Hsum = 0;
-    for (int l = 0; l < a.nlayer; ++l) {
-        Hmax = Hmax > a.H[l] ? Hmax : a.H[l];
-        Hsum += a.H[l];
+    NetTrainMulti m;
+    int warp_floats = 0;
+    for (int k = 0; k < count; ++k) {
+        const NetTrainArgs& a = m.a[k] = args[k];
+        int Hmax = a.D, Hsum = 0;
+        for (int l = 0; l < a.nlayer; ++l) {
+            Hmax = Hmax > a.H[l] ? Hmax : a.H[l];
+            Hsum += a.H[l];
+        }
+        const int wf = kTrainAtoms * (2 * a.D + 2 * Hsum + 2 * Hmax);
+        warp_floats = warp_floats > wf ? warp_floats : wf;
     }
-    const int warp_floats = kTrainAtoms * (2 * a.D + 2 * Hsum + 2 * Hmax);
     int wpc = 4;
     while (wpc > 1 && (size_t)wpc * warp_floats * sizeof(float) > 200 * 1024) --wpc;
     const size_t sm = sizeof(float) * (size_t)warp_floats * wpc;
@@ -1146,7 +1177,7 @@ cudaError_t launch_net_train(const NetTrainArgs& a, cudaStream_t st) {
         lim = (int)sm;
     }
     const int per_block = kTrainAtoms * wpc;
-    k_net_train<<<(n + per_block - 1) / per_block, 32 * wpc, sm, st>>>(a, warp_floats);
+    k_net_train<<<dim3((n + per_block - 1) / per_block, count), 32 * wpc, sm, st>>>(m, warp_floats);
     return cudaGetLastError();
 }
 

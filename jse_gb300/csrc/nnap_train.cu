@@ -16,7 +16,9 @@
 namespace nnapgb {
 namespace {
 
-constexpr int kTrainChunk = 256;  // slots per partial sum
+// Slots per partial sum: few atoms take short chunks, so that their sums run on more CTAs (2600
+// atoms: 55 -> 17 us), many the long ones, whose partials are a quarter of the memory.
+int train_chunk(int n) { return n <= 32768 ? 64 : 256; }
 
 int net_params(const Species& sp) {
     int p = 0, in = sp.D;
@@ -99,7 +101,7 @@ void train_enqueue(nnap_handle* h, const Batch& B, const double* bE, const doubl
         tiles[t] = grad_tiles(m.sp[t]);
         tmax = std::max(tmax, (int)tiles[t].size());
     }
-    const int nchunk = (n + kTrainChunk - 1) / kTrainChunk;
+    const int nchunk = (n + train_chunk(n) - 1) / train_chunk(n);
     h->tu.ensure((size_t)n1 * h->fp_stride);
     h->trec.ensure((size_t)n1 * Vmax);
     h->tpart.ensure((size_t)T * std::max(nchunk, 1) * Pmax);
@@ -213,7 +215,8 @@ void train_enqueue(nnap_handle* h, const Batch& B, const double* bE, const doubl
             }
         }
     }
-    // network passes, one launch per species
+    // network passes, all species in one launch
+    std::vector<NetTrainArgs> nets;
     for (int t = 0; t < T && n > 0; ++t) {
         const NetDev& nd = h->nets[t];
         NetTrainArgs a;
@@ -234,16 +237,17 @@ void train_enqueue(nnap_handle* h, const Batch& B, const double* bE, const doubl
         a.V = Vmax;
         a.gfp = want_w ? h->tgfp.p : nullptr;
         a.dfp = want_w ? h->tdfp.p : nullptr;
-        CK(launch_net_train(a, st));
-        ++h->launches;
+        nets.push_back(a);
     }
+    CK(launch_net_train(nets.data(), (int)nets.size(), st));
+    ++h->launches;
     // chunk partials and their FP64 sums
     ReduceArgs ra;
     std::memset(&ra, 0, sizeof ra);
     ra.range = h->type_start.p;
     ra.T = T;
     ra.rec = h->trec.p;
-    ra.chunk = kTrainChunk;
+    ra.chunk = train_chunk(n);
     ra.nchunk = nchunk;
     ra.partial = h->tpart.p;
     ra.Pmax = Pmax;

@@ -91,7 +91,8 @@ struct ReduceArgs {
 cudaError_t upload_sh_constants_train();
 cudaError_t launch_train_prep(const double* bF, int n, float4* bFf, cudaStream_t st);
 cudaError_t launch_jvp(int kind, int lmax, int np, int n1, const JvpArgs& a, cudaStream_t st);
-cudaError_t launch_net_train(const NetTrainArgs& a, cudaStream_t st);
+// count species in one launch; a[k].t names the species.
+cudaError_t launch_net_train(const NetTrainArgs* a, int count, cudaStream_t st);
 cudaError_t launch_train_reduce(const ReduceArgs& a, cudaStream_t st);
 cudaError_t launch_wgrad(int kind, int lmax, int np, int n1, const WgradArgs& a, cudaStream_t st);
 // out[e] = sum over w < G of partial[w * per + e] (FP64, in w order), e < per.

@@ -133,3 +133,33 @@ def test_network_slices(T, nmax, hidden, n):
     with NNAP(model) as p:
         for a, b in zip(p.calEnergyForceVirialsBatch([small, s]), [p.calEnergyForceVirials(small), p.calEnergyForceVirials(s)]):
             assert np.array_equal(a["energies"], b["energies"]) and np.array_equal(a["forces"], b["forces"])
+
+
+@pytest.mark.parametrize("n", [1, 31, 40, 65, 700])
+def test_training_sums(n):
+    """Parameter gradients with fewer partials than the final sum's rows, chunks of a few slots and
+    several, against the oracle's energies: dL/d(output bias) is the sum of the upstream energy
+    gradients times sigma_E, exactly (2^-24 sqrt(n) of its terms), and the radial weights' gradient
+    of a batch is the sum of its structures' (the FP32 partials' 2^-22)."""
+    from jse_gb300.nnap import NNAP
+    rng = np.random.default_rng(n)
+    basis = {"type": "spherical_chebyshev", "nmax": 4, "lmax": 4, "rcut": 5.0, "wtype": "fuse", "fuse_size": 2,
+             "fuse_weight": rng.normal(0, 1, 4).tolist()}
+    model = W.write_model(["A", "B"], dict(basis, wtype="default"), [8, 8], 1)
+    for m in model["models"]:
+        m["basis"] = basis
+    ss = [W.random_liquid(n, 0.05, [0.5, 0.5], 1.9, n), W.random_liquid(12, 0.05, [0.5, 0.5], 1.9, 3)]
+    N = n + 12
+    be, bf = rng.normal(0, 1, N), rng.normal(0, 1, (N, 3))
+    with NNAP(model) as p:
+        both = p.backwardEnergyForceBatch(ss, be, bf, want_fp=True)
+        one = [p.backwardEnergyForceBatch([ss[0]], be[:n], bf[:n], want_fp=True),
+               p.backwardEnergyForceBatch([ss[1]], be[n:], bf[n:], want_fp=True)]
+    types = np.concatenate([s.types for s in ss])
+    for t in range(2):
+        want = be[types == t + 1].sum()
+        assert abs(both["grad_nn"][t][-1] - want) <= 1e-6 * np.abs(be).sum()
+        for key in ("grad_nn", "grad_fp"):
+            parts = one[0][key][t] + one[1][key][t]
+            size = np.abs(one[0][key][t]) + np.abs(one[1][key][t])
+            assert np.abs(both[key][t] - parts).max() <= 1e-5 * max(size.max(), 1e-30)
