@@ -224,7 +224,7 @@ struct nnap_handle {
     nnapgb::DevBuf<int> spos, scount;
     int M = 0;
     // LAMMPS-style boundary: caller's atoms (local + ghost), list, targets of the scatter
-    nnapgb::DevBuf<double> lmp_x, lmp_forces, lmp_virials;
+    nnapgb::DevBuf<double> lmp_x, lmp_forces, lmp_virials, lmp_vpart;
     nnapgb::Pinned lmp_pin_in, lmp_pin_out;  // per-call layout arrays in, results out
     // the list on the device from the last LAMMPS call (reused with nlflag = 0)
     bool lmp_cached = false;

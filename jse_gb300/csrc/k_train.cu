@@ -1018,7 +1018,7 @@ __global__ void __launch_bounds__(32 * kWgWarps) k_wgrad(WgradArgs g) {
 // A CTA per 8 entries, 32 rows of threads: row r adds partials r, r + 32, .. and the 32 sums are
 // added in order, in FP64.  Few entries per CTA spread the FP64 additions, whose pipe takes two
 // per cycle and SM, over more SMs.  2600 partials of 200 entries: one thread per entry through
-// all partials 320 us, 32 entries per CTA 45, 8 entries 25.
+// all partials 320 us, 32 entries per CTA 45, 8 entries 15.
 constexpr int kFinalRows = 32, kFinalCols = 8;
 
 __global__ void __launch_bounds__(kFinalCols * kFinalRows) k_wgrad_final(const float* __restrict__ partial, int G, int per,

@@ -18,7 +18,7 @@ __global__ void k_lmp_rows(int, int, const int*, const int*, const int*, const d
 __global__ void k_lmp_count(PairBufs, int, int*);
 __global__ void k_lmp_fill(PairBufs, int, const int*, int*, int*);
 __global__ void k_lmp_gather(PairBufs, int, const int*, const int*, const int*, double*, double*);
-__global__ void k_lmp_virial_sum(const double*, int, double*);
+__global__ void k_lmp_virial_sum(const double*, int, int, int, double*);
 }  // namespace nnapgb
 
 using namespace nnapgb;
@@ -27,6 +27,7 @@ namespace {
 constexpr int kLmpNeighMask = 0x1FFFFFFF;  // LAMMPS keeps special-bond bits above this mask
 constexpr size_t kLmpThreadedEntries = 1 << 18;  // list entries from which the copy is threaded
 constexpr unsigned kLmpMaxThreads = 8;
+constexpr int kLmpSumRows = 512;  // atoms per CTA of the global-virial sum
 }
 
 namespace {
@@ -126,6 +127,7 @@ int compute_lammps(nnap_handle* h, int nlflag, int inum, int nall, const int* il
         h->lmp_tlist.ensure(std::max<size_t>(total, 1));
         h->lmp_forces.ensure(3 * (size_t)nall);
         h->lmp_virials.ensure(9 * (size_t)nall);
+        h->lmp_vpart.ensure(6 * ((size_t)nall / kLmpSumRows + 1));
         cudaStream_t st = h->stream;
         const int T = h->model.ntypes();
         CK(cudaMemcpyAsync(h->lmp_x.p, x, sizeof(double) * 3 * nall, cudaMemcpyHostToDevice, st));
@@ -166,7 +168,7 @@ int compute_lammps(nnap_handle* h, int nlflag, int inum, int nall, const int* il
         }
         k_sort_cells<<<(unsigned)(((size_t)nall * 32 + 255) / 256), 256, 0, st>>>(h->lmp_tstart.p, nall,
                                                                                   h->lmp_tlist.p);
-        k_lmp_gather<<<(nall + 127) / 128, 128, 0, st>>>(pair_bufs(h), nall, h->lmp_rowof.p, h->lmp_tstart.p,
+        k_lmp_gather<<<(unsigned)(((size_t)nall * 8 + 127) / 128), 128, 0, st>>>(pair_bufs(h), nall, h->lmp_rowof.p, h->lmp_tstart.p,
                                                          h->lmp_tlist.p, h->lmp_forces.p, h->lmp_virials.p);
         h->launches += 3;
         CK(cudaGetLastError());
@@ -174,8 +176,10 @@ int compute_lammps(nnap_handle* h, int nlflag, int inum, int nall, const int* il
         // summed on the device in a fixed order
         const bool per_atom_v = vflag_atom || cvflag_atom;
         if (vflag && !per_atom_v) {
-            k_lmp_virial_sum<<<1, kLmpSumThreads, 0, st>>>(h->lmp_virials.p, nall, h->virial.p);
-            ++h->launches;
+            const int chunks = (nall + kLmpSumRows - 1) / kLmpSumRows;
+            k_lmp_virial_sum<<<chunks, kLmpSumThreads, 0, st>>>(h->lmp_virials.p, 9, nall, kLmpSumRows, h->lmp_vpart.p);
+            k_lmp_virial_sum<<<1, kLmpSumThreads, 0, st>>>(h->lmp_vpart.p, 6, chunks, chunks, h->virial.p);
+            h->launches += 2;
             CK(cudaGetLastError());
         }
         const size_t out_bytes = al(sizeof(double) * 3 * nall) + al(sizeof(double) * n1) +
