@@ -43,6 +43,8 @@ __global__ void k_gather(PairBufs, int, const int*, double*, double*);
 __global__ void k_reduce_chunks(const int*, const int*, const double*, const double*, double*);
 __global__ void k_reduce_structs(const int*, int, const double*, double*, double*);
 
+__global__ void k_pack_results(PackArgs);
+
 // Launch shapes chosen per atom-count bucket by the autotuner (defaults below).
 struct Tuning {
     int desc_fwd_warps = 4;  // warps per CTA of the descriptor forward kernels
@@ -240,6 +242,12 @@ struct nnap_handle {
     nnapgb::DevBuf<nnapgb::GradTile> ttiles;
     int GS = 0;                  // cell-offset groups per atom + 1 kept by k_neighbors (0: none)
     nnapgb::DevBuf<int> gstart;  // [n][GS] group starts of each neighbour row
+    // small host calls: inputs through one pinned buffer and device array, results through one
+    // mapped buffer; pack_flags: the outputs wanted by the call in progress (0: not packed)
+    nnapgb::Pinned pin_in, pin_out;
+    nnapgb::DevBuf<char> dev_in;
+    int pack_flags = 0;
+    int pack_off[5] = {-1, -1, -1, -1, -1};
     int* h_status = nullptr;  // pinned: [0]=err bits [1]=max count [2..]=type_start
     bool profiling = false;
     cudaEvent_t order_ev = nullptr;

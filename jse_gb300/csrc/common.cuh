@@ -62,4 +62,14 @@ struct PairBufs {
     int GS;                // groups per atom + 1 (largest offset count of the batch + 1), or 0
 };
 
+// Results of a small host call packed into mapped host memory (k_pack_results): offsets of
+// energy, energies, forces, virial and virials in doubles (-1: not wanted).
+struct PackArgs {
+    int off[5] = {-1, -1, -1, -1, -1};
+    int nstruct = 0, n = 0;
+    const double *energy = nullptr, *e_atom = nullptr, *forces = nullptr, *virial = nullptr, *virials = nullptr;
+    const int* orig = nullptr;
+    double* out = nullptr;
+};
+
 }  // namespace nnapgb

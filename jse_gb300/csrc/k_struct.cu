@@ -254,6 +254,23 @@ __global__ void k_unpermute(const double* __restrict__ in, const int* __restrict
     if (k < n) out[orig[k]] = in[k];
 }
 
+// The requested results of a small host call into one mapped host buffer (PackArgs::out, offsets
+// in doubles; -1: not wanted), per-atom energies back in atom order.
+__global__ void k_pack_results(PackArgs p) {
+    pdl_enter();
+    const int step = gridDim.x * blockDim.x, t = blockIdx.x * blockDim.x + threadIdx.x;
+    auto copy = [&](int off, const double* src, int count) {
+        if (off >= 0)
+            for (int k = t; k < count; k += step) p.out[off + k] = src[k];
+    };
+    copy(p.off[0], p.energy, p.nstruct);
+    copy(p.off[3], p.virial, 9 * p.nstruct);
+    if (p.off[1] >= 0)
+        for (int k = t; k < p.n; k += step) p.out[p.off[1] + (p.orig ? p.orig[k] : k)] = p.e_atom[k];
+    copy(p.off[2], p.forces, 3 * p.n);
+    copy(p.off[4], p.virials, 9 * p.n);
+}
+
 // Shared memory of one warp; SLOTS stencil cells are held at a time (all of them where the
 // structure has at most SLOTS).
 template <int SLOTS, int NA>

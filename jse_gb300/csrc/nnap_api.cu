@@ -794,6 +794,26 @@ void enqueue(nnap_handle* h, const Batch& B, const double* d_x, const int* d_typ
     CK(cudaMemcpyAsync(h->h_status, h->status.p, sizeof(int) * 2, cudaMemcpyDeviceToHost, st));
 }
 
+// Queue the packing of a small host call's results (after the sequence, outside its graph: the
+// outputs wanted may change from call to call).
+void enqueue_pack(nnap_handle* h, const Batch& B) {
+    if (!h->pack_flags) return;
+    PackArgs p;
+    std::copy(h->pack_off, h->pack_off + 5, p.off);
+    p.nstruct = B.nstruct;
+    p.n = B.natoms;
+    p.energy = h->energy.p;
+    p.e_atom = h->e_atom.p;
+    p.forces = h->forces.p;
+    p.virial = h->virial.p;
+    p.virials = h->virials.p;
+    p.orig = h->renumbered ? h->orig.p : nullptr;
+    p.out = static_cast<double*>(h->pin_out.p);
+    const int work = std::max(B.natoms * 4, B.nstruct * 9);
+    CK(launch_pdl(k_pack_results, dim3(std::max(1, std::min((work + 255) / 256, h->sm_count))), dim3(256), 0, h->stream, p));
+    ++h->launches;
+}
+
 // Identity of a launch sequence: what the captured graph depends on.
 std::vector<long long> layout_key(nnap_handle* h, const Batch& B, const double* d_x, const int* d_type, bool fp_only) {
     std::vector<long long> k = {B.nstruct, B.natoms, B.ncells, h->M, (long long)(intptr_t)d_x,
@@ -947,6 +967,7 @@ void evaluate(nnap_handle* h, const Batch& B, const double* d_x, const int* d_ty
         } else {
             enqueue(h, B, d_x, d_type, fp_only);
         }
+        enqueue_pack(h, B);
         CK(cudaStreamSynchronize(h->stream));
         ++h->layout_runs;
         const int bits = h->h_status[0];
@@ -959,6 +980,7 @@ void evaluate(nnap_handle* h, const Batch& B, const double* d_x, const int* d_ty
                 h->tuned[tune_bucket] = tune_launches(h, B, d_x, d_type);
                 // the outputs of this call come from the chosen shapes
                 enqueue(h, B, d_x, d_type, fp_only);
+                enqueue_pack(h, B);
                 CK(cudaStreamSynchronize(h->stream));
                 h->last_layout = layout_key(h, B, nullptr, nullptr, fp_only);
                 h->layout_runs = 1;
@@ -1011,6 +1033,49 @@ void upload_inputs(nnap_handle* h, int n, const double* x, const int* type) {
         CK(cudaMemcpyAsync(h->x.p, x, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, h->stream));
         CK(cudaMemcpyAsync(h->type.p, type, sizeof(int) * n, cudaMemcpyHostToDevice, h->stream));
     }
+}
+
+// A host call of at most kHostStage bytes in and out goes through pinned memory: one copy in, and
+// results written into mapped memory by the last kernel of the sequence, so the call has one
+// synchronisation and no pageable copies, whose fixed cost outweighs their bytes: 33 atoms 196 ->
+// 147 us, 4099 atoms 311 -> 259, 25000 atoms (1.5 MB) 559 -> 548.  Larger calls copy directly.
+constexpr size_t kHostStage = 2 << 20;
+
+size_t host_bytes(const Batch& B, int flags) {
+    const size_t n = B.natoms, S = B.nstruct;
+    size_t d = 0;
+    if (flags & NNAP_WANT_ENERGY) d += S;
+    if (flags & NNAP_WANT_ENERGIES) d += n;
+    if (flags & NNAP_WANT_FORCES) d += 3 * n;
+    if (flags & NNAP_WANT_VIRIAL) d += 9 * S;
+    if (flags & NNAP_WANT_VIRIALS) d += 9 * n;
+    return sizeof(double) * d + (3 * sizeof(double) + sizeof(int)) * n;
+}
+
+void compute_staged(nnap_handle* h, const Batch& B, const double* x, const int* type, int flags, const Outputs& o) {
+    const size_t n = B.natoms, xb = 3 * sizeof(double) * n, tb = sizeof(int) * n;
+    const size_t len[5] = {(size_t)B.nstruct, n, 3 * n, 9 * (size_t)B.nstruct, 9 * n};
+    const int bit[5] = {NNAP_WANT_ENERGY, NNAP_WANT_ENERGIES, NNAP_WANT_FORCES, NNAP_WANT_VIRIAL, NNAP_WANT_VIRIALS};
+    double* const dst[5] = {o.energy, o.energies, o.forces, o.virial, o.virials};
+    size_t total = 0;
+    for (int k = 0; k < 5; ++k) {
+        h->pack_off[k] = flags & bit[k] ? (int)total : -1;
+        if (flags & bit[k]) total += len[k];
+    }
+    char* in = static_cast<char*>(h->pin_in.ensure(xb + tb));
+    const double* out = static_cast<const double*>(h->pin_out.ensure(sizeof(double) * std::max<size_t>(total, 1)));
+    h->dev_in.ensure(xb + tb);
+    std::memcpy(in, x, xb);
+    std::memcpy(in + xb, type, tb);
+    CK(cudaMemcpyAsync(h->dev_in.p, in, xb + tb, cudaMemcpyHostToDevice, h->stream));
+    struct Packing {
+        int& f;
+        ~Packing() { f = 0; }
+    } packing{h->pack_flags};
+    h->pack_flags = flags;
+    evaluate(h, B, reinterpret_cast<const double*>(h->dev_in.p), reinterpret_cast<const int*>(h->dev_in.p + xb), false);
+    for (int k = 0; k < 5; ++k)
+        if (flags & bit[k]) std::memcpy(dst[k], out + h->pack_off[k], sizeof(double) * len[k]);
 }
 
 }  // namespace nnapgb
@@ -1150,6 +1215,9 @@ int nnap_destroy(nnap_handle* h) {
     for (auto* b : {&h->lmp_x, &h->lmp_forces, &h->lmp_virials, &h->lmp_vpart}) b->release();
     h->lmp_pin_in.release();
     h->lmp_pin_out.release();
+    h->pin_in.release();
+    h->pin_out.release();
+    h->dev_in.release();
     for (auto* b : {&h->lmp_type, &h->lmp_ilist, &h->lmp_off, &h->lmp_idx, &h->lmp_rowtype, &h->lmp_rowof,
                     &h->lmp_tcount, &h->lmp_tstart, &h->lmp_tfill, &h->lmp_tlist})
         b->release();
@@ -1236,6 +1304,10 @@ int nnap_compute_batch(nnap_handle* h, int nstruct, const int* natoms, const dou
         h->launches = 0;
         const Batch& B = plan_batch(h, nstruct, natoms, box_kind, boxes);
         if (B.natoms && (!x || !type)) throw ApiFail(NNAP_ERR_ARG, "positions or types are NULL");
+        if (B.natoms && flags && host_bytes(B, flags) <= kHostStage) {
+            compute_staged(h, B, x, type, flags, o);
+            return NNAP_OK;
+        }
         upload_inputs(h, B.natoms, x, type);
         evaluate(h, B, h->x.p, h->type.p, false);
         copy_out(h, B, flags, o, cudaMemcpyDeviceToHost);

@@ -163,3 +163,31 @@ def test_training_sums(n):
             parts = one[0][key][t] + one[1][key][t]
             size = np.abs(one[0][key][t]) + np.abs(one[1][key][t])
             assert np.abs(both[key][t] - parts).max() <= 1e-5 * max(size.max(), 1e-30)
+
+
+@pytest.mark.parametrize("n", [7, 15000, 22000])
+def test_host_staging(n):
+    """Host calls that go through pinned staging (up to 2 MiB in and out) and ones that copy directly
+    give the same numbers for every choice of outputs, with outputs in any order, call after call."""
+    import ctypes as C
+    from jse_gb300 import nnap as J
+    model = W.write_model(["A"], {"type": "chebyshev", "nmax": 3, "rcut": 3.0}, [4], 1)
+    s = W.random_liquid(n, 0.05, [1.0], 1.6, n)
+    with J.NNAP(model) as p:
+        ref = p.calEnergyForceVirials(s)  # n = 22000 with per-atom virials: above the limit
+        shapes = {"energy": (1,), "energies": (n,), "forces": (n, 3), "virial": (9,), "virials": (n, 9)}
+        for flags in (J.WANT_ENERGY, J.WANT_FORCES, J.WANT_ENERGIES | J.WANT_VIRIAL, 31, J.WANT_VIRIALS, 31):
+            out = {k: np.full(v, np.nan) for k, v in shapes.items()}
+            p._check(p._L.nnap_compute(p._handle(), n, J._dptr(np.ascontiguousarray(s.x)), J._iptr(s.types), s.box_kind,
+                                       J._dptr(np.ascontiguousarray(s.box.reshape(9))), flags,
+                                       *[J._dptr(out[k]) for k in ("energy", "energies", "forces", "virial", "virials")]))
+            for bit, k in zip((1, 2, 4, 8, 16), ("energy", "energies", "forces", "virial", "virials")):
+                if flags & bit:
+                    assert np.array_equal(out[k].reshape(-1), np.reshape(ref[k], -1)), (flags, k)
+                else:
+                    assert np.isnan(out[k]).all()
+        bad = W.Structure(s.x, s.types.copy(), s.box, s.box_kind)
+        bad.types[-1] = 2
+        with pytest.raises(ValueError):
+            p.calForces(bad)
+        assert np.array_equal(p.calForces(s), ref["forces"])
