@@ -44,6 +44,8 @@ __global__ void k_reduce_chunks(const int*, const int*, const double*, const dou
 __global__ void k_reduce_structs(const int*, int, const double*, double*, double*);
 
 __global__ void k_pack_results(PackArgs);
+size_t order_small_bytes(int n, int ncells, int T);
+cudaError_t launch_order_small(const OrderArgs& a, cudaStream_t st);
 
 // Launch shapes chosen per atom-count bucket by the autotuner (defaults below).
 struct Tuning {
@@ -319,8 +321,9 @@ PairBufs pair_bufs(nnap_handle* h);
 void ensure_work(nnap_handle* h, int n, int nstruct, int ncells, int nchunks);
 // Queue the species sort of n rows (slots ordered by species, stable).
 void enqueue_species(nnap_handle* h, int n, const int* d_type);
-// Queue the species sort of the batch's atoms and the mirror index of the pair rows.
-void enqueue_species_mirror(nnap_handle* h, const Batch& B, const int* d_type);
+// Queue the species sort of the batch's atoms (unless the cell ordering did it) and the mirror
+// index of the pair rows.
+void enqueue_species_mirror(nnap_handle* h, const Batch& B, const int* d_type, bool species_done = false);
 // Queue descriptors, networks and descriptor gradients; with gather, also the
 // force / virial gather over mirrored rows and the per-structure reductions.
 // orig: the atom of each row when the rows are in cell order (forces and virials are

@@ -72,4 +72,18 @@ struct PackArgs {
     double* out = nullptr;
 };
 
+// One-CTA ordering of a small evaluation (k_order_small).
+constexpr int kOrderAtoms = 1024;  // most atoms (one per thread)
+constexpr int kOrderCells = 4096;  // and most cells
+struct OrderArgs {
+    int n, ncells, T;
+    bool renumber;
+    const int *cell_of, *type;
+    const float4 *xf, *xlo;
+    const double* xw;
+    int *cell_start, *cell_atoms, *cell_of2, *type2, *orig, *perm, *type_start;
+    float4 *xfc, *xloc;
+    double* xw2;
+};
+
 }  // namespace nnapgb

@@ -60,7 +60,7 @@ __global__ void k_wrap_bin(const StructDev* __restrict__ S, const int* __restric
     }
     const int cid = st.c0 + c[0] + st.nc[0] * (c[1] + st.nc[1] * c[2]);
     cell_of[i] = cid;
-    atomicAdd(&cell_count[cid], 1);
+    if (cell_count) atomicAdd(&cell_count[cid], 1);
 }
 
 // Exclusive scan of n ints by one CTA of 1024 threads; out has n + 1 entries.  A thread takes
@@ -245,6 +245,133 @@ __global__ void __launch_bounds__(256) k_renumber(int* __restrict__ cell_atoms, 
     type2[k] = type[a];
     orig[k] = a;
     cell_atoms[k] = k;
+}
+
+// The cell order, the renumbering and the species order of a small evaluation by one CTA, an
+// atom per thread: the work of k_scan_excl, k_fill_cells, k_sort_cells, k_renumber (or
+// k_cell_order) and the species sort, with the same results.  Each of those takes 2 to 4 us of
+// latency whatever its size: the stage of 33 atoms 47 -> 40 us, of 500 atoms 52 -> 44.  (With
+// several atoms per thread the one CTA's loads take longer than the launches: 2000 atoms 54
+// against 51, 4000 atoms 73 against 59.)
+__global__ void __launch_bounds__(kOrderAtoms) k_order_small(OrderArgs a) {
+    pdl_enter();
+    extern __shared__ int osm[];
+    __shared__ int s_warp[32], s_tot[kMaxTypes + 1];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, n = a.n, C = a.ncells, T = a.T;
+    int* cnt = osm;                               // [C + 1] counts, then starts
+    int* list = osm + C + 1;                      // [n] atoms by cell, in no order inside a cell
+    int* wc = list + n;                           // [ceil(n / 32)][T] species counts of 32 rows
+    uint8_t* stype = reinterpret_cast<uint8_t*>(wc + ((n + 31) / 32) * T);  // [n] species of each row
+    for (int c = tid; c <= C; c += kOrderAtoms) cnt[c] = 0;
+    // this thread's atom
+    const bool have = tid < n;
+    int cell = 0, rk = 0, t = 0;
+    float4 f = make_float4(0.f, 0.f, 0.f, 0.f), lo = f;
+    double x0 = 0.0, x1 = 0.0, x2 = 0.0;
+    if (have) {
+        cell = a.cell_of[tid];
+        t = a.type[tid];
+        f = a.xf[tid];
+        lo = a.xlo[tid];
+        if (a.renumber) {
+            x0 = a.xw[3 * tid];
+            x1 = a.xw[3 * tid + 1];
+            x2 = a.xw[3 * tid + 2];
+        }
+    }
+    __syncthreads();
+    if (have) rk = atomicAdd(&cnt[cell], 1);
+    __syncthreads();
+    {  // exclusive scan of the counts, in place: consecutive cells per thread
+        const int per = (C + kOrderAtoms) / kOrderAtoms, b = min(C + 1, tid * per), e = min(C + 1, b + per);
+        int own = 0;
+        for (int c = b; c < e; ++c) own += cnt[c];
+        int s = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += u;
+        }
+        if (lane == 31) s_warp[w] = s;
+        __syncthreads();
+        int tot = s_warp[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, tot, o);
+            if (lane >= o) tot += u;
+        }
+        const int before = w ? __shfl_sync(0xffffffffu, tot, w - 1) : 0;
+        int x = before + s - own;
+        for (int c = b; c < e; ++c) {
+            const int v = cnt[c];
+            cnt[c] = x;
+            a.cell_start[c] = x;
+            x += v;
+        }
+    }
+    __syncthreads();
+    if (have) list[cnt[cell] + rk] = tid;
+    __syncthreads();
+    if (have) {
+        const int b = cnt[cell], e = cnt[cell + 1];
+        int r = b;  // the atom's place: its rank by index in its cell
+        for (int q = b; q < e; ++q) r += list[q] < tid ? 1 : 0;
+        a.xfc[r] = f;
+        a.xloc[r] = lo;
+        if (a.renumber) {
+            a.xw2[3 * r] = x0;
+            a.xw2[3 * r + 1] = x1;
+            a.xw2[3 * r + 2] = x2;
+            a.cell_of2[r] = cell;
+            a.type2[r] = t;
+            a.orig[r] = tid;
+            a.cell_atoms[r] = r;
+        } else {
+            a.cell_atoms[r] = tid;
+        }
+        stype[a.renumber ? r : tid] = t >= 1 && t <= T ? (uint8_t)(t - 1) : 255;
+    }
+    __syncthreads();
+    // species order, stable: counts per 32 rows, their sums before each, then the ranks
+    const int ty = have ? stype[tid] : 255;
+    unsigned mine = 0;
+    if (tid - lane < n)
+        for (int q = 0; q < T; ++q) {
+            const unsigned m = __ballot_sync(0xffffffffu, ty == q);
+            if (lane == 0) wc[w * T + q] = __popc(m);
+            if (ty == q) mine = m;
+        }
+    __syncthreads();
+    if (w < T) {  // kMaxTypes <= 32 warps, and at most 32 groups of rows
+        const int v = lane * 32 < n ? wc[lane * T + w] : 0;
+        int s = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += u;
+        }
+        if (lane * 32 < n) wc[lane * T + w] = s - v;
+        if (lane == 31) s_tot[w] = s;
+    }
+    __syncthreads();
+    int base = 0;
+    for (int q = 0; q < T; ++q) {
+        if (tid == 0) a.type_start[q] = base;
+        if (q == ty) a.perm[base + wc[w * T + q] + __popc(mine & ((1u << lane) - 1u))] = tid;
+        base += s_tot[q];
+    }
+    if (tid == 0) a.type_start[T] = base;
+}
+
+// Shared memory of k_order_small, or 0 when the evaluation is not one for it.
+size_t order_small_bytes(int n, int ncells, int T) {
+    if (n < 1 || n > kOrderAtoms || ncells > kOrderCells) return 0;
+    return sizeof(int) * ((size_t)ncells + 1 + n + (size_t)((n + 31) / 32) * T) + ((n + 15) & ~15);
+}
+
+cudaError_t launch_order_small(const OrderArgs& a, cudaStream_t st) {
+    const size_t sm = order_small_bytes(a.n, a.ncells, a.T);  // at most 24 KB
+    return launch_pdl(k_order_small, dim3(1), dim3(kOrderAtoms), sm, st, a);
 }
 
 // out[orig[k]] = in[k]: a per-atom array of a cell-ordered evaluation back in atom order.

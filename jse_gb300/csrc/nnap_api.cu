@@ -537,40 +537,72 @@ void prepare_layout(nnap_handle* h, const Batch& B) {
     CK(cudaStreamSynchronize(st));
 }
 
+// One CTA orders the atoms by cell and by species (k_order_small) where there is one per thread.
+bool order_small(const Batch& B, int T) { return order_small_bytes(B.natoms, B.ncells, T) > 0; }
+
 // Cell list and neighbour rows of every atom of the batch (cutoff and cell grid from
 // the structure descriptors already on the device).
 void enqueue_neighbors(nnap_handle* h, const Batch& B, const double* d_x, const int* d_type, bool renumber) {
     const int n = B.natoms;
     const int T = h->model.ntypes();
     cudaStream_t st = h->stream;
-    CK(cudaMemsetAsync(h->cell_count.p, 0, sizeof(int) * B.ncells, st));
-    CK(cudaMemsetAsync(h->cell_fill.p, 0, sizeof(int) * B.ncells, st));
+    const int nw = h->tune.nb_warps;
+    const bool small = order_small(B, T);
+    if (!small) {
+        CK(cudaMemsetAsync(h->cell_count.p, 0, sizeof(int) * B.ncells, st));
+        CK(cudaMemsetAsync(h->cell_fill.p, 0, sizeof(int) * B.ncells, st));
+    }
     if (n > 0) {
-        CK(launch_pdl(k_wrap_bin, dim3((n + 255) / 256), dim3(256), 0, st, h->sdev.p, h->sid.p, d_x, d_type, n, T, h->xw.p, h->xf.p,
-                                                    h->xlo.p, h->cell_of.p, h->cell_count.p, h->status.p));
+        CK(launch_pdl(k_wrap_bin, dim3((n + 255) / 256), dim3(256), 0, st, h->sdev.p, h->sid.p, d_x, d_type, n, T, h->xw.p,
+                      h->xf.p, h->xlo.p, h->cell_of.p, small ? nullptr : h->cell_count.p, h->status.p));
         ++h->launches;
     }
-    CK(launch_pdl(k_scan_excl, dim3(1), dim3(1024), 0, st, h->cell_count.p, B.ncells, h->cell_start.p));
-    ++h->launches;
-    if (n > 0) {
-        CK(launch_pdl(k_fill_cells, dim3((n + 255) / 256), dim3(256), 0, st, h->cell_of.p, n, h->cell_start.p, h->cell_fill.p, h->cell_atoms.p));
-        CK(launch_pdl(k_sort_cells, dim3((B.ncells * 32 + 255) / 256), dim3(256), 0, st, h->cell_start.p, B.ncells, h->cell_atoms.p));
-        const int nw = h->tune.nb_warps;
-        if (renumber) {  // the rest of the evaluation numbers atoms in cell order
-            CK(launch_pdl(k_renumber, dim3((n + 255) / 256), dim3(256), 0, st, h->cell_atoms.p, n, h->xf.p, h->xlo.p,
-                          h->xw.p, h->cell_of.p, d_type, h->xfc.p, h->xloc.p, h->xw2.p, h->cell_of2.p, h->type2.p,
-                          h->orig.p));
-            CK(launch_neighbors(h->sdev.p, h->sid.p, h->xw2.p, h->xfc.p, h->xloc.p, h->cell_of2.p, h->cell_start.p,
-                                h->cell_atoms.p, n, B.max_off, nw, h->sm_count, pair_bufs(h), h->status.p, h->status.p + 1,
-                                st));
-        } else {
-            CK(launch_pdl(k_cell_order, dim3((n + 255) / 256), dim3(256), 0, st, h->cell_atoms.p, n, h->xf.p, h->xlo.p,
-                          h->xfc.p, h->xloc.p));
-            CK(launch_neighbors(h->sdev.p, h->sid.p, h->xw.p, h->xfc.p, h->xloc.p, h->cell_of.p, h->cell_start.p,
-                                h->cell_atoms.p, n, B.max_off, nw, h->sm_count, pair_bufs(h), h->status.p, h->status.p + 1,
-                                st));
+    if (small) {  // the species order too
+        OrderArgs a;
+        a.n = n;
+        a.ncells = B.ncells;
+        a.T = T;
+        a.renumber = renumber;
+        a.cell_of = h->cell_of.p;
+        a.type = d_type;
+        a.xf = h->xf.p;
+        a.xlo = h->xlo.p;
+        a.xw = h->xw.p;
+        a.cell_start = h->cell_start.p;
+        a.cell_atoms = h->cell_atoms.p;
+        a.cell_of2 = h->cell_of2.p;
+        a.type2 = h->type2.p;
+        a.orig = h->orig.p;
+        a.perm = h->perm.p;
+        a.type_start = h->type_start.p;
+        a.xfc = h->xfc.p;
+        a.xloc = h->xloc.p;
+        a.xw2 = h->xw2.p;
+        CK(launch_order_small(a, st));
+        ++h->launches;
+    } else {
+        CK(launch_pdl(k_scan_excl, dim3(1), dim3(1024), 0, st, h->cell_count.p, B.ncells, h->cell_start.p));
+        ++h->launches;
+        if (n > 0) {
+            CK(launch_pdl(k_fill_cells, dim3((n + 255) / 256), dim3(256), 0, st, h->cell_of.p, n, h->cell_start.p,
+                          h->cell_fill.p, h->cell_atoms.p));
+            CK(launch_pdl(k_sort_cells, dim3((B.ncells * 32 + 255) / 256), dim3(256), 0, st, h->cell_start.p, B.ncells,
+                          h->cell_atoms.p));
+            if (renumber)  // the rest of the evaluation numbers atoms in cell order
+                CK(launch_pdl(k_renumber, dim3((n + 255) / 256), dim3(256), 0, st, h->cell_atoms.p, n, h->xf.p, h->xlo.p,
+                              h->xw.p, h->cell_of.p, d_type, h->xfc.p, h->xloc.p, h->xw2.p, h->cell_of2.p, h->type2.p,
+                              h->orig.p));
+            else
+                CK(launch_pdl(k_cell_order, dim3((n + 255) / 256), dim3(256), 0, st, h->cell_atoms.p, n, h->xf.p, h->xlo.p,
+                              h->xfc.p, h->xloc.p));
+            h->launches += 3;
         }
-        h->launches += 4;
+    }
+    if (n > 0) {
+        CK(launch_neighbors(h->sdev.p, h->sid.p, renumber ? h->xw2.p : h->xw.p, h->xfc.p, h->xloc.p,
+                            renumber ? h->cell_of2.p : h->cell_of.p, h->cell_start.p, h->cell_atoms.p, n, B.max_off, nw,
+                            h->sm_count, pair_bufs(h), h->status.p, h->status.p + 1, st));
+        ++h->launches;
     }
 }
 
@@ -585,10 +617,10 @@ void enqueue_species(nnap_handle* h, int n, const int* d_type) {
     h->launches += 3;
 }
 
-void enqueue_species_mirror(nnap_handle* h, const Batch& B, const int* d_type) {
+void enqueue_species_mirror(nnap_handle* h, const Batch& B, const int* d_type, bool species_done) {
     const int n = B.natoms;
     if (n <= 0) return;
-    enqueue_species(h, n, d_type);
+    if (!species_done) enqueue_species(h, n, d_type);
     CK(launch_pdl(k_mirror, dim3((unsigned)(((size_t)n * 32 + 255) / 256)), dim3(256), 0, h->stream, 
         h->sdev.p, h->sid.p, pair_bufs(h), n, h->status.p));
     ++h->launches;
@@ -787,7 +819,7 @@ void enqueue(nnap_handle* h, const Batch& B, const double* d_x, const int* d_typ
     h->renumbered = renumber;
     enqueue_neighbors(h, B, d_x, d_type, renumber);
     const int* dt = renumber ? h->type2.p : d_type;
-    enqueue_species_mirror(h, B, dt);
+    enqueue_species_mirror(h, B, dt, order_small(B, h->model.ntypes()));
     h->mark(1);
     enqueue_eval(h, B, dt, fp_only, true, renumber ? h->orig.p : nullptr);
     CK(cudaGetLastError());

@@ -191,3 +191,24 @@ def test_host_staging(n):
         with pytest.raises(ValueError):
             p.calForces(bad)
         assert np.array_equal(p.calForces(s), ref["forces"])
+
+
+@pytest.mark.parametrize("T,n,density,tilt", [
+    (1, 1, 0.01, None), (3, 2, 0.02, 0.1), (16, 31, 0.05, None), (16, 33, 0.05, 0.1), (3, 1023, 0.05, None),
+    (3, 1024, 0.05, 0.1), (3, 1025, 0.05, None), (2, 900, 0.0002, None), (2, 900, 0.0001, None)])
+def test_one_cta_order(T, n, density, tilt):
+    """Atoms ordered by one CTA (up to 1024 atoms and 4096 cells) and by the general kernels: exact
+    neighbour sets, descriptors in atom order, and the structure alone equal to it in a batch too
+    large for one CTA, bit for bit."""
+    from jse_gb300.nnap import NNAP
+    basis = {"type": "chebyshev", "nmax": 2, "rcut": 5.0, "wtype": "none"}
+    model = W.write_model(["S%d" % k for k in range(T)], basis, [4], 1)
+    s = W.random_liquid(n, density, [1.0 / T] * T, 1.9, n, tilt=tilt)
+    other = W.random_liquid(1100, 0.05, [1.0 / T] * T, 1.9, 5)
+    ref = ON.compute(OM.load(model), s.x, s.types, s.box_kind, s.box, want_fp=True)
+    with NNAP(model) as p:
+        _same_rows(p, s, 5.0)
+        assert np.abs(p.calFp(s) - ref["fp"]).max() <= 1e-5 * max(1.0, np.abs(ref["fp"]).max())
+        alone, batch = p.calEnergyForceVirials(s), p.calEnergyForceVirialsBatch([s, other], per_atom_virial=True)[0]
+        for key in ("energies", "forces", "virials"):
+            assert np.array_equal(alone[key], batch[key])
