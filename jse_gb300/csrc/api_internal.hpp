@@ -40,7 +40,7 @@ __global__ void k_type_hist(const int*, int, int, int*);
 __global__ void k_type_offsets(int*, int, int, int*);
 __global__ void k_type_scatter(const int*, int, int, const int*, int*);
 __global__ void k_gather(PairBufs, int, const int*, double*, double*);
-__global__ void k_reduce_chunks(const int*, const int*, const double*, const double*, double*);
+__global__ void k_reduce_chunks(const int*, const int*, const double*, const double*, double*, double*, double*);
 __global__ void k_reduce_structs(const int*, int, const double*, double*, double*);
 
 __global__ void k_pack_results(PackArgs);

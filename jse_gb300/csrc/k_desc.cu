@@ -295,13 +295,13 @@ struct SphFNShape {
 // thread per channel (1500 warp instructions per atom; the shared-memory path is 75 % busy).
 template <int L, int NP, int N1>
 __global__ void __launch_bounds__(32 * kDescMaxWarps) k_sph_fwd_n(DescArgs a) {
-    pdl_enter();
     using S = SphFNShape<L, NP, N1>;
     extern __shared__ float smem[];
     const int T = a.T;
     const int ntab = T * kFwdTypes * NP;  // alpha[tc][tn][p], zero for tn >= T
     float* sAl = smem;
     for (int q = threadIdx.x; q < ntab; q += blockDim.x) sAl[q] = a.fwd_alpha[q];
+    pdl_enter();  // alpha belongs to the model
     __syncthreads();
     const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int w = blockIdx.x * (blockDim.x >> 5) + wl;
@@ -667,7 +667,6 @@ __device__ __forceinline__ void bwd_columns(const float* __restrict__ gh, const 
 constexpr int kBwdWarps = 4;  // most warps per CTA
 template <int L, int NP, int N1, int LPA>
 __global__ void __launch_bounds__(32 * kBwdWarps, LPA == 32 ? 5 : 6) k_sph_bwd_n(DescArgs a) {
-    pdl_enter();
     using S = SphNShape<L, NP, N1>;
     constexpr int APW = 32 / LPA;
     extern __shared__ __align__(16) float smem[];
@@ -701,6 +700,7 @@ __global__ void __launch_bounds__(32 * kBwdWarps, LPA == 32 ? 5 : 6) k_sph_bwd_n
         sN[s] = make_float2(n0.x, l1 <= L ? n1.x : 0.f);
         sCo[s] = make_float2(l0 < a.nl2 ? n0.z : 0.f, l1 <= L && l1 < a.nl2 ? n1.z : 0.f);
     }
+    pdl_enter();  // the tables above belong to the model: only what follows needs the previous kernel
     __syncthreads();
     const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane / LPA, sub = lane % LPA;
     const int w0 = (blockIdx.x * (blockDim.x >> 5) + wl) * APW, w = w0 + grp;

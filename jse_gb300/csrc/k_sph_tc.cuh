@@ -134,7 +134,6 @@ __device__ __forceinline__ void tmem_ld_halves_wait(uint32_t taddr, float* v) {
 
 template <int L, int NP, int N1>
 __global__ void __launch_bounds__(32 * kFwdTcWarps, 4) k_sph_fwd_tc(DescArgs a) {
-    pdl_enter();
     using S = SphTcShape<L, NP>;
     constexpr int KM = S::KM, NPN = S::NPN;
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -155,6 +154,8 @@ __global__ void __launch_bounds__(32 * kFwdTcWarps, 4) k_sph_fwd_tc(DescArgs a) 
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc::smem_u32(&mbar[q])) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    // alpha belongs to the model; TMEM is taken after the previous kernel (which may hold it) ends
+    pdl_enter();
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(&s_tmem)),
                      "r"(32 * kFwdTcWarps)

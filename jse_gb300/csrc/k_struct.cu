@@ -779,8 +779,10 @@ cudaError_t launch_neighbors(const StructDev* S, const int* sid, const double* x
 // Mirror index: for entry (i -> j, image n) the position of (j -> i, image -n) in j's row.
 // Rows are ordered by (cell-offset group, atom index); the mirrored entry lies in group
 // noff-1-g of j's row (the negated cell offset).  With group starts kept, it is found
-// by a scan of that group (a few entries); otherwise by binary search on (group, atom).
-// One warp per row.
+// in that group: halved by atom number to a few entries (a small box has tens of one image),
+// which are read two at a time; otherwise by binary search on (group, atom).  One warp per row.
+// Bound: the chain of dependent loads.  Reading a group's entries one after another took 14 us
+// at 33 atoms and 549 on the 1M-atom glass, now 7 and 529 (1024-structure batch 402 -> 335).
 __global__ void k_mirror(const StructDev* __restrict__ S, const int* __restrict__ sid, PairBufs P, int n,
                          int* __restrict__ err) {
     pdl_enter();
@@ -805,12 +807,20 @@ __global__ void k_mirror(const StructDev* __restrict__ S, const int* __restrict_
         int found = -1;
         if (groups) {
             const int* gs = P.gstart + (size_t)j * P.GS;
-            const int lo = min(gs[want_g], cj), hi = min(gs[want_g + 1], cj);
-            for (int q = lo; q < hi; ++q)
-                if (row[q] == target) {
-                    found = q;
-                    break;
-                }
+            int lo = min(gs[want_g], cj);
+            const int hi = min(gs[want_g + 1], cj);
+            int len = hi - lo;
+            while (len > 4) {  // the first entry whose atom is not below i stays within [lo, lo + len]
+                const int half = len >> 1;
+                const bool below = (int)(row[lo + half] >> 32) < i;
+                lo = below ? lo + half + 1 : lo;
+                len = below ? len - half - 1 : half;
+            }
+            for (int q = lo; q < hi && found < 0; q += 2) {
+                const uint64_t v0 = row[q], v1 = q + 1 < hi ? row[q + 1] : 0;
+                if (v0 == target) found = q;
+                if (v1 == target) found = q + 1;
+            }
         } else {
             const uint16_t* grow = P.grp + (size_t)j * M;
             const uint64_t want = ((uint64_t)(uint32_t)want_g << 32) | (uint32_t)i;
@@ -919,7 +929,10 @@ __global__ void k_type_scatter(const int* __restrict__ type, int n, int T, const
 // of the row as float-float pairs (exact products, error-free additions); the partial sums
 // are combined by a fixed xor butterfly, so the result does not depend on timing.
 // Own-row loads are coalesced; only g of the mirrored entry is a scattered load.  Four
-// lanes per atom (eight atoms per warp) beat eight: 0.416 -> 0.347 ms on the batch.
+// lanes per atom (eight atoms per warp) beat eight: 0.416 -> 0.347 ms on the batch's scatter
+// stage.  Bound: HBM (the row, its mirror index and two gradients per entry); for few atoms the
+// chain of loads and the instruction fetch, so the loop holds one entry and loads ahead:
+// 286 -> 267 us on the batch, 455 -> 437 on the 1M-atom glass, 25 -> 18 on 4000 copper atoms.
 constexpr int kGatherLanes = 4;
 
 __device__ __forceinline__ void ff_merge(float& h, float& l, unsigned mask, int off) {
@@ -945,36 +958,40 @@ __global__ void k_gather(PairBufs P, int n, const int* __restrict__ orig, double
 #pragma unroll
     for (int d = 0; d < 9; ++d) { vh[d] = 0.f; vl[d] = 0.f; }
     const size_t row = (size_t)a * M;
-    // two entries per step: both mirrored-gradient loads (an index load, then a gather) are
-    // in flight before either is used; the second entry's terms are added after the first's,
-    // so the summation order is that of one entry per step
-    for (int k0 = sub; k0 < cnt; k0 += 2 * kGatherLanes) {
-        const int k1 = k0 + kGatherLanes;
-        const bool two = k1 < cnt;
-        const int r0 = P.rev[row + k0], r1 = two ? P.rev[row + k1] : r0;
-        const float4 gr0 = P.g[r0], gr1 = P.g[r1];
-        const float4 go0 = P.g[row + k0], go1 = two ? P.g[row + k1] : go0;
-        const float4 dn0 = P.dx[row + k0], dn1 = two ? P.dx[row + k1] : dn0;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            if (h == 1 && !two) break;
-            const float4 go = h ? go1 : go0;
-            const float4 dn = h ? dn1 : dn0;
-            const float4 gr = h ? gr1 : gr0;
-            const float dx = -dn.x, dy = -dn.y, dz = -dn.z;
-            ff_acc(fh[0], fl[0], gr.x); ff_acc(fh[0], fl[0], -go.x);
-            ff_acc(fh[1], fl[1], gr.y); ff_acc(fh[1], fl[1], -go.y);
-            ff_acc(fh[2], fl[2], gr.z); ff_acc(fh[2], fl[2], -go.z);
-            ff_acc_prod(vh[0], vl[0], dx, gr.x);
-            ff_acc_prod(vh[1], vl[1], dy, gr.y);
-            ff_acc_prod(vh[2], vl[2], dz, gr.z);
-            ff_acc_prod(vh[3], vl[3], dx, gr.y);
-            ff_acc_prod(vh[4], vl[4], dx, gr.z);
-            ff_acc_prod(vh[5], vl[5], dy, gr.z);
-            ff_acc_prod(vh[6], vl[6], dy, gr.x);
-            ff_acc_prod(vh[7], vl[7], dz, gr.x);
-            ff_acc_prod(vh[8], vl[8], dz, gr.y);
+    // one entry per step, the next one's three loads and the mirror index of the one after it in
+    // flight meanwhile
+    constexpr int S = kGatherLanes;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 gr = zero, go = zero, dn = zero;
+    int rn = 0;
+    if (sub < cnt) {
+        gr = P.g[P.rev[row + sub]];
+        go = P.g[row + sub];
+        dn = P.dx[row + sub];
+        if (sub + S < cnt) rn = P.rev[row + sub + S];
+    }
+#pragma unroll 1
+    for (int k = sub; k < cnt; k += S) {
+        const float4 cr = gr, co = go, cd = dn;
+        if (k + S < cnt) {
+            gr = P.g[rn];
+            go = P.g[row + k + S];
+            dn = P.dx[row + k + S];
+            if (k + 2 * S < cnt) rn = P.rev[row + k + 2 * S];
         }
+        const float dx = -cd.x, dy = -cd.y, dz = -cd.z;
+        ff_acc(fh[0], fl[0], cr.x); ff_acc(fh[0], fl[0], -co.x);
+        ff_acc(fh[1], fl[1], cr.y); ff_acc(fh[1], fl[1], -co.y);
+        ff_acc(fh[2], fl[2], cr.z); ff_acc(fh[2], fl[2], -co.z);
+        ff_acc_prod(vh[0], vl[0], dx, cr.x);
+        ff_acc_prod(vh[1], vl[1], dy, cr.y);
+        ff_acc_prod(vh[2], vl[2], dz, cr.z);
+        ff_acc_prod(vh[3], vl[3], dx, cr.y);
+        ff_acc_prod(vh[4], vl[4], dx, cr.z);
+        ff_acc_prod(vh[5], vl[5], dy, cr.z);
+        ff_acc_prod(vh[6], vl[6], dy, cr.x);
+        ff_acc_prod(vh[7], vl[7], dz, cr.x);
+        ff_acc_prod(vh[8], vl[8], dz, cr.y);
     }
 #pragma unroll
     for (int off = kGatherLanes / 2; off > 0; off >>= 1) {
@@ -993,12 +1010,14 @@ __global__ void k_gather(PairBufs P, int n, const int* __restrict__ orig, double
 }
 
 // ----------------------------------------------------------------- per-structure totals
-// chunk c covers atoms [cb[c], ce[c]); partial[c][0] = sum E, partial[c][1..9] = sum W.
+// chunk c covers atoms [cb[c], ce[c]); partial[c][0] = sum E, partial[c][1..9] = sum W.  Where
+// every structure is one chunk, energy and virial (else NULL) receive the totals at once.
 constexpr int kRedBlock = 256;
 
 __global__ void k_reduce_chunks(const int* __restrict__ cb, const int* __restrict__ ce,
                                 const double* __restrict__ e_atom, const double* __restrict__ virials,
-                                double* __restrict__ partial) {
+                                double* __restrict__ partial, double* __restrict__ energy,
+                                double* __restrict__ virial) {
     pdl_enter();
     __shared__ double sm[10][kRedBlock / 32];
     const int c = blockIdx.x;
@@ -1020,7 +1039,9 @@ __global__ void k_reduce_chunks(const int* __restrict__ cb, const int* __restric
     if (threadIdx.x < 10) {
         double t = 0.0;
         for (int q = 0; q < kRedBlock / 32; ++q) t += sm[threadIdx.x][q];
-        partial[10 * (size_t)c + threadIdx.x] = t;
+        if (!energy) partial[10 * (size_t)c + threadIdx.x] = t;
+        else if (threadIdx.x == 0) energy[c] = t;
+        else virial[9 * (size_t)c + threadIdx.x - 1] = t;
     }
 }
 

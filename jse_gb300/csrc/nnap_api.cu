@@ -792,14 +792,19 @@ void enqueue_eval(nnap_handle* h, const Batch& B, const int* d_type, bool fp_onl
             ++h->launches;
         }
         const int nchunks = (int)B.cb.size();
+        // every structure one chunk (none empty): its totals in one launch
+        bool single = nchunks == B.nstruct;
+        for (int q = 0; single && q < B.nstruct; ++q) single = B.sc[q] == q;
         if (nchunks) {
-            CK(launch_pdl(k_reduce_chunks, dim3(nchunks), dim3(kRedBlock), 0, st, h->chunk_b.p, h->chunk_e.p, h->e_atom.p, h->virials.p,
-                                                            h->partial.p));
+            CK(launch_pdl(k_reduce_chunks, dim3(nchunks), dim3(kRedBlock), 0, st, h->chunk_b.p, h->chunk_e.p, h->e_atom.p,
+                          h->virials.p, h->partial.p, single ? h->energy.p : nullptr, single ? h->virial.p : nullptr));
             ++h->launches;
         }
-        CK(launch_pdl(k_reduce_structs, dim3((B.nstruct * 32 + 127) / 128), dim3(128), 0, st, h->struct_chunks.p, B.nstruct, h->partial.p,
-                                                                        h->energy.p, h->virial.p));
-        ++h->launches;
+        if (!single) {
+            CK(launch_pdl(k_reduce_structs, dim3((B.nstruct * 32 + 127) / 128), dim3(128), 0, st, h->struct_chunks.p, B.nstruct,
+                          h->partial.p, h->energy.p, h->virial.p));
+            ++h->launches;
+        }
     }
     h->mark(5);
 }
