@@ -50,7 +50,8 @@ bool net_tc_prepare(const Species& sp, NetTC& tc, std::string& why);
 void net_tc_release(NetTC& tc);
 // One launch over nt consecutive species a[k].t = a[0].t + k, all with the same layout.
 // err receives ERRBIT_TIMEOUT if a bounded wait on the tensor cores gave up.
-// split: threads per tile row in the epilogues (2 or 4).
+// split: threads per tile row in the epilogues (2 or 4) where a CTA has one tile in flight; two
+// tiles in flight take 2 each.  The results do not depend on it.
 cudaError_t launch_net_tc(const NetArgs* a, const NetTC* const* tc, int nt, int* err, int sm_count, int split,
                           cudaStream_t st);
 

@@ -15,6 +15,9 @@ __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// The wait alone: the next kernel launches when this one has ended.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Launch with the programmatic-stream-serialization attribute (captured into CUDA graphs
 // as a programmatic dependency).
 template <typename... KArgs, typename... Args>

@@ -212,3 +212,23 @@ def test_one_cta_order(T, n, density, tilt):
         alone, batch = p.calEnergyForceVirials(s), p.calEnergyForceVirialsBatch([s, other], per_atom_virial=True)[0]
         for key in ("energies", "forces", "virials"):
             assert np.array_equal(alone[key], batch[key])
+
+
+@pytest.mark.parametrize("T,nmax,hidden,n", [
+    (1, 10, (16,), 1999), (2, 15, (64, 64), 1921), (3, 18, (32, 48, 20), 2047), (2, 12, (64, 100), 2048),
+    (1, 8, (250, 96), 1700)])
+def test_network_two_tiles(T, nmax, hidden, n):
+    """The tensor-core network with two tiles in flight (more than two per SM): one to three hidden
+    layers, descriptors and layers of odd widths, short last tiles of every species, two groups
+    that fit and (250-96) do not.  The same operations in the same order as with one tile in
+    flight: equal to the structures alone, bit by bit, and those to the oracle within the mixed
+    path's 5e-5 eV, 1e-3 and 2e-4 of the largest force."""
+    from jse_gb300.nnap import NNAP
+    model = _model({"type": "chebyshev", "nmax": nmax, "rcut": 5.0}, T, hidden)
+    ss = [W.random_liquid(k, 0.05, [1.0 / T] * T, 1.9, k) for k in (n, 13, 1, 130)]
+    _check(model, ss[3], "mixed", 5e-5, 1e-3, 2e-4)
+    with NNAP(model, precision="mixed") as p:
+        alone = [p.calEnergyForceVirials(s) for s in ss]
+        for k, b in enumerate(p.calEnergyForceVirialsBatch(ss * 24)):
+            a = alone[k % 4]
+            assert np.array_equal(a["energies"], b["energies"]) and np.array_equal(a["forces"], b["forces"])
