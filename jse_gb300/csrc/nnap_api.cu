@@ -630,8 +630,8 @@ void enqueue_eval(nnap_handle* h, const Batch& B, const int* d_type, bool fp_onl
     const int n = B.natoms;
     const int T = h->model.ntypes();
     cudaStream_t st = h->stream;
-    if (n > 0) CK(cudaMemsetAsync(h->fp.p, 0, sizeof(float) * (size_t)n * h->fp_stride, st));
-    // descriptors, per run of species sharing a basis shape and per sub-basis
+    // descriptors, per run of species sharing a basis shape and per sub-basis; the kernels write
+    // every column of a row's descriptor, and what is beyond it is read by none
     // compact rows for the sub-bases that scan them (once per evaluation)
     bool sub_built = false;
     auto descriptors = [&](bool fwd) {
@@ -787,7 +787,9 @@ void enqueue_eval(nnap_handle* h, const Batch& B, const int* d_type, bool fp_onl
     if (!fp_only && gather) {
         if (n > 0) {
             const int gb = h->tune.gather_block;  // threads per CTA, four per atom
-            CK(launch_pdl(k_gather, dim3((unsigned)(((size_t)n * 4 + gb - 1) / gb)), dim3(gb), 0, st, pair_bufs(h), n,
+            // the whole L1 for the scattered gradients: 32000 atoms 517 -> 505 us, 400 thousand 5393 -> 5374,
+            // 4000 and fewer the same
+            CK(launch_after(k_gather, dim3((unsigned)(((size_t)n * 4 + gb - 1) / gb)), dim3(gb), 0, st, pair_bufs(h), n,
                           orig, h->forces.p, h->virials.p));
             ++h->launches;
         }

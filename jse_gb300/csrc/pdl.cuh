@@ -35,4 +35,17 @@ cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t sme
     return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
+// Launch after the previous kernel has ended.  A kernel that is let in early starts on an SM
+// next to the last blocks of the one before and keeps that SM's split between shared memory
+// and L1 for its whole run; a large grid that wants another split is better launched so.
+template <typename... KArgs, typename... Args>
+cudaError_t launch_after(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+
 }  // namespace nnapgb

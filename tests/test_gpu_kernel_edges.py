@@ -232,3 +232,24 @@ def test_network_two_tiles(T, nmax, hidden, n):
         for k, b in enumerate(p.calEnergyForceVirialsBatch(ss * 24)):
             a = alone[k % 4]
             assert np.array_equal(a["energies"], b["energies"]) and np.array_equal(a["forces"], b["forces"])
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp32"])
+@pytest.mark.parametrize("basis", [
+    {"type": "chebyshev", "nmax": 6, "rcut": 5.0},
+    {"type": "spherical_chebyshev", "nmax": 8, "lmax": 6, "rcut": 6.0},
+    {"type": "spherical_chebyshev", "nmax": 3, "lmax": 4, "l3max": 4, "l4max": 2, "rcut": 5.0},
+    {"type": "merge", "basis": [{"type": "chebyshev", "nmax": 5, "rcut": 6.0},
+                                {"type": "spherical_chebyshev", "nmax": 3, "lmax": 3, "rcut": 4.5, "wtype": "full"}]}])
+def test_descriptors_after_another_structure(precision, basis):
+    """Rows of descriptors are written whole: what an evaluation before left in the workspace does
+    not show, and atoms without a neighbour have zeros.  Equal bit by bit."""
+    from jse_gb300.nnap import NNAP
+    from tests.golden.make_golden import _model as make
+    model = make(["A", "B"], basis, [8, 8], 2)
+    big, s = W.random_liquid(300, 0.06, [0.5, 0.5], 1.9, 1), W.random_liquid(7, 0.002, [0.5, 0.5], 1.9, 5)
+    with NNAP(model, precision=precision) as p, NNAP(model, precision=precision) as q:
+        p.calEnergyForceVirials(big)
+        a, b = p.calEnergyForceVirials(s), q.calEnergyForceVirials(s)
+        assert np.array_equal(p.calFp(s), q.calFp(s)) and np.isfinite(p.calFp(s)).all()
+        assert all(np.array_equal(a[k], b[k]) for k in ("energies", "forces", "virials"))
