@@ -236,7 +236,9 @@ int nnap_set_graphs(nnap_handle* h, int on);
  * the caller's own batch (warps per CTA 2/4/8 of the descriptor forward, descriptor
  * backward and neighbour kernels; 64/128/256 threads per CTA of the gather; 2 or 4
  * threads per row of the tensor-core network) and keeps the fastest; later evaluations
- * of the bucket reuse them.  Off by default; untuned buckets use 4, 4, 4, 128, 4. */
+ * of the bucket reuse them.  Off by default; untuned buckets use 4, 4, 4, 128, 4.  The
+ * backward of the compiled spherical shapes runs at most 4 warps (8 means 4), and the network
+ * 2 threads per row where a CTA has two tiles in flight. */
 int nnap_set_autotune(nnap_handle* h, int on);
 /* Shapes used for natoms atoms: [descriptor forward warps, descriptor backward warps,
  * neighbour warps, gather threads, network threads per row]; *tuned = 1 when the

@@ -7,9 +7,12 @@
 //   -> k_renumber (energy/force evaluations: atoms in cell order from here on; descriptor-
 //      only calls take k_cell_order and keep atom order) -> k_neighbors
 //   -> species sort (k_type_hist, k_type_offsets, k_type_scatter) -> k_mirror
+//      (up to 1024 atoms k_order_small does all between k_wrap_bin and k_neighbors and the
+//      species sort)
 //   -> descriptor forward (per run of species sharing a basis shape, per sub-basis)
 //   -> network per species -> descriptor backward -> k_gather -> k_reduce_chunks
-//   -> k_reduce_structs, then one host synchronisation (neighbour capacity, error bits).
+//   -> k_reduce_structs (left out where every structure is one chunk), for host calls of
+//   up to 2 MiB k_pack_results, then one host synchronisation (neighbour capacity, error bits).
 #include <cuda_runtime.h>
 
 #include <algorithm>
