@@ -33,12 +33,12 @@
 // Within a tile: the sigmoid has no branch, silu' is kept instead of formed again, two values
 // are split per conversion, a row's sectors are loaded whole and four at a time, and the next
 // tile's rows are called into L2.  Before and now: 909 -> 403 us for 1048573 atoms
-// (90-64-64-1, two species), 498 -> 232 us for 400 thousand (126-64-64-1, three species);
+// (90-64-64-1, two species), 498 -> 232 us for 488206 (126-64-64-1, three species);
 // with one group 524 and 279.
 //
 // The next kernel is not let in early: its blocks would start on an SM as soon as the tile
 // kernel's one block there ends, and keep the SM's split between shared memory and L1, which
-// with 160 to 226 KiB of operands leaves the backward kernels little L1 (400 thousand atoms:
+// with 160 to 226 KiB of operands leaves the backward kernels little L1 (488206 atoms:
 // 5399 us per evaluation, 5947 with the early launch; 32000 atoms 525 against 531).
 // Shared-memory operands use the no-swizzle K-major canonical layout: 8x8 core
 // matrices of 128 bytes, adjacent in K at LBO = 128 bytes and in M/N at

@@ -751,7 +751,7 @@ static cudaError_t launch_nb(const StructDev* S, const int* sid, const double* x
     }
     const dim3 grid((unsigned)((n + warps * NA - 1) / (warps * NA))), block(32 * warps);
     // the kernels before have no shared memory: with many atoms each SM takes its split anew
-    // (1048573 atoms 7159 -> 7078 us, 400 thousand 5393 -> 5387, fewer the same)
+    // (1048573 atoms 7159 -> 7078 us, 488206 5393 -> 5387, fewer the same)
     if (NA == 8)
         return launch_after(k_neighbors<SLOTS, NA>, grid, block, smem, st, S, sid, xw, xfc, xloc, cell_of, cell_start,
                             cell_atoms, n, P, err, max_count);

@@ -790,7 +790,7 @@ void enqueue_eval(nnap_handle* h, const Batch& B, const int* d_type, bool fp_onl
     if (!fp_only && gather) {
         if (n > 0) {
             const int gb = h->tune.gather_block;  // threads per CTA, four per atom
-            // the whole L1 for the scattered gradients: 32000 atoms 517 -> 505 us, 400 thousand 5393 -> 5374,
+            // the whole L1 for the scattered gradients: 32000 atoms 517 -> 505 us, 488206 5393 -> 5374,
             // 4000 and fewer the same
             CK(launch_after(k_gather, dim3((unsigned)(((size_t)n * 4 + gb - 1) / gb)), dim3(gb), 0, st, pair_bufs(h), n,
                           orig, h->forces.p, h->virials.p));
