@@ -177,13 +177,16 @@ void put_operand(std::vector<uint8_t>& img, int byte_off, int R, int K, F&& M) {
 
 // 1/(1 + e^-z) without the branch of a division, so that the 16 units of a step overlap: the
 // machine's approximate reciprocal and one step of Newton's iteration, which leaves the
-// rounding of the last operation.  The denominator stops at 2^126, where silu(z) is below
-// 1e-36; a NaN of z reaches the results through their factor z.
+// rounding of the last operation.  Below -87.3, where the denominator nears 2^126 and its
+// reciprocal the smallest normal number, it is zero (silu is within 2e-36 of it there, and silu
+// and silu' stay zero however large -z is, as with a division).  Infinities and NaN of z reach
+// the results as they do with a division.
 __device__ __forceinline__ float sigmoidf_(float z) {
-    const float y = fminf(1.f + expf(-z), 8.507059e37f);
+    const float y = 1.f + expf(-z);
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
-    return fmaf(r, fmaf(-y, r, 1.f), r);
+    r = fmaf(r, fmaf(-y, r, 1.f), r);
+    return z < -87.3f ? 0.f : r;
 }
 
 // Species t0 .. t0+nt-1 of one launch; all share one layout.  Tiles are numbered species
