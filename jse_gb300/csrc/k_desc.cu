@@ -25,6 +25,7 @@
 
 #include "common.cuh"
 #include "pdl.cuh"
+#include "smem_limit.cuh"
 #include "desc.cuh"
 #include "sph_math.cuh"
 #include "k_sph_tc.cuh"
@@ -1118,14 +1119,8 @@ cudaError_t launch_invariants(const InvArgs& a, bool fwd, cudaStream_t st) {
     if (a.nmax <= 0 || a.ncol <= 0) return cudaSuccess;
     const int grid = (int)(((long long)a.nmax * a.NP + kInvThreads - 1) / kInvThreads);
     const size_t sm = sizeof(float) * kInvThreads * (a.K | 1) * (fwd ? 1 : 2);
-    static int limit_fwd = 0, limit_bwd = 0;  // raised once, before any graph capture
-    int& lim = fwd ? limit_fwd : limit_bwd;
-    if ((int)sm > lim && sm > 48 * 1024) {
-        const cudaError_t e = fwd ? cudaFuncSetAttribute(k_inv_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)
-                                  : cudaFuncSetAttribute(k_inv_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        lim = (int)sm;
-    }
+    const cudaError_t e = allow_smem(fwd ? k_inv_fwd : k_inv_bwd, sm);
+    if (e != cudaSuccess) return e;
     if (fwd) return launch_pdl(&k_inv_fwd, dim3(grid), dim3(kInvThreads), sm, st, a);
     return launch_pdl(&k_inv_bwd, dim3(grid), dim3(kInvThreads), sm, st, a);
 }
@@ -1140,15 +1135,8 @@ cudaError_t launch_radial(const DescArgs& a, bool fwd, cudaStream_t st) {
     const int wpc = a.warps;
     const int grid = (n + wpc - 1) / wpc;
     const size_t sm = sizeof(float) * a.T * a.T * NP * Fuse<N1>::N1P;
-    static int limit_fwd = 0, limit_bwd = 0;  // raised once, before any graph capture
-    int& lim = fwd ? limit_fwd : limit_bwd;
-    if ((int)sm > lim && sm > 48 * 1024) {
-        const cudaError_t e =
-            fwd ? cudaFuncSetAttribute(k_radial_fwd<NP, N1, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)
-                : cudaFuncSetAttribute(k_radial_bwd<NP, N1, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        lim = (int)sm;
-    }
+    const cudaError_t e = fwd ? allow_smem(k_radial_fwd<NP, N1, RB>, sm) : allow_smem(k_radial_bwd<NP, N1, RB>, sm);
+    if (e != cudaSuccess) return e;
     if (fwd) return launch_pdl(&k_radial_fwd<NP, N1, RB>, dim3(grid), dim3(32 * wpc), sm, st, a);
     return launch_pdl(&k_radial_bwd<NP, N1, RB>, dim3(grid), dim3(32 * wpc), sm, st, a);
 }
@@ -1165,13 +1153,8 @@ cudaError_t launch_sph_bwd_lanes(const DescArgs& a, cudaStream_t st) {
     const size_t sm = sizeof(float) * (fixed + (size_t)wpc * S::warp_floats(a.T, APW, diag));
     if (sm > 227 * 1024) return cudaErrorInvalidValue;
     const int grid = (a.nmax + wpc * APW - 1) / (wpc * APW);
-    static int lim = 0;
-    if ((int)sm > lim) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(k_sph_bwd_n<L, NP, N1, LPA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        lim = (int)sm;
-    }
+    const cudaError_t e = allow_smem(k_sph_bwd_n<L, NP, N1, LPA>, sm);
+    if (e != cudaSuccess) return e;
     return launch_pdl(&k_sph_bwd_n<L, NP, N1, LPA>, dim3(grid), dim3(32 * wpc), sm, st, a);
 }
 
@@ -1194,13 +1177,8 @@ cudaError_t launch_sph_fwd_n(const DescArgs& a, cudaStream_t st) {
     const int grid = (a.nmax + wpc - 1) / wpc;
     const size_t sm = sizeof(float) * (((size_t)a.T * kFwdTypes * NP + 3) / 4 * 4 + (size_t)wpc * S::WARP_FLOATS);
     if (sm > 227 * 1024) return cudaErrorInvalidValue;
-    static int lim = 0;
-    if ((int)sm > lim) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(k_sph_fwd_n<L, NP, N1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        lim = (int)sm;
-    }
+    const cudaError_t e = allow_smem(k_sph_fwd_n<L, NP, N1>, sm);
+    if (e != cudaSuccess) return e;
     return launch_pdl(&k_sph_fwd_n<L, NP, N1>, dim3(grid), dim3(32 * wpc), sm, st, a);
 }
 
@@ -1221,17 +1199,8 @@ cudaError_t launch_sph(const DescArgs& a, bool fwd, cudaStream_t st) {
     const int grid = (n + wpc - 1) / wpc;
     const size_t wbytes = sizeof(float) * ((size_t)a.T * a.T * NP * Fuse<N1>::N1P);
     const size_t sm = wbytes + sizeof(float) * wpc * (fwd ? S::FWD_WARP_FLOATS : S::BWD_WARP_FLOATS);
-    // the shared-memory limit is raised once per kernel (before any graph capture: the
-    // first evaluation of a layout always runs eagerly)
-    static int limit_fwd = 0, limit_bwd = 0;
-    int& lim = fwd ? limit_fwd : limit_bwd;
-    if ((int)sm > lim) {
-        const cudaError_t e =
-            fwd ? cudaFuncSetAttribute(k_sph_fwd<L, NP, N1, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)
-                : cudaFuncSetAttribute(k_sph_bwd<L, NP, N1, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        lim = (int)sm;
-    }
+    const cudaError_t e = fwd ? allow_smem(k_sph_fwd<L, NP, N1, RB>, sm) : allow_smem(k_sph_bwd<L, NP, N1, RB>, sm);
+    if (e != cudaSuccess) return e;
     if (fwd) return launch_pdl(&k_sph_fwd<L, NP, N1, RB>, dim3(grid), dim3(32 * wpc), sm, st, a);
     return launch_pdl(&k_sph_bwd<L, NP, N1, RB>, dim3(grid), dim3(32 * wpc), sm, st, a);
 }

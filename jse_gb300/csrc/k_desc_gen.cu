@@ -2,9 +2,8 @@
 // bases and spherical bases of every expansion degree L = 0 .. 12, for the NNAP and NEP
 // radial functions.  A launch uses as many warps per CTA as its launch shape asks for and
 // shared memory allows (one atom slot per warp).
-#include <map>
-
 #include "k_desc_gen.cuh"
+#include "smem_limit.cuh"
 
 namespace nnapgb {
 
@@ -25,15 +24,8 @@ cudaError_t launch_g(Kern kern, const DescArgs& a, size_t per_warp, int np, int 
     while (wpc > 1 && per_warp * wpc > kSmemMax) wpc >>= 1;
     const size_t sm = per_warp * wpc;
     if (sm > kSmemMax) return cudaErrorInvalidValue;
-    // the shared-memory limit is raised once per kernel and size (the first evaluation of a
-    // layout runs eagerly, before any graph capture)
-    static std::map<const void*, size_t> limits;
-    size_t& lim = limits[reinterpret_cast<const void*>(kern)];
-    if (sm > 48 * 1024 && sm > lim) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        lim = sm;
-    }
+    const cudaError_t e = allow_smem(kern, sm);
+    if (e != cudaSuccess) return e;
     const int grid = (a.nmax + wpc - 1) / wpc;
     return launch_pdl(kern, dim3(grid), dim3(32 * wpc), sm, st, a, np, n1);
 }

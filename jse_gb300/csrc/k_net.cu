@@ -21,6 +21,7 @@
 //   mu[D] | 1/sigma[D] | for each layer: W^T[in][H] | W[H][in] | b[H] | w_out[H_L] | b_out
 #include "desc.cuh"
 #include "pdl.cuh"
+#include "smem_limit.cuh"
 
 namespace nnapgb {
 namespace {
@@ -466,31 +467,19 @@ cudaError_t launch_net_fp32(const NetArgs* args, int count, int sms, cudaStream_
     const size_t sm = sizeof(float) * (size_t)wf * wpc;
     const int per_block = kNetAtoms * wpc;
     if (count == 1 && !deep) {
-        static size_t limit = 48 * 1024;
-        if (sm > limit) {
-            const cudaError_t e = cudaFuncSetAttribute(k_net_fp32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            if (e != cudaSuccess) return e;
-            limit = sm;
-        }
+        const cudaError_t e = allow_smem(k_net_fp32, sm);
+        if (e != cudaSuccess) return e;
         return launch_pdl(&k_net_fp32, dim3((n + per_block - 1) / per_block), dim3(32 * wpc), sm, st, args[0], wf);
     }
     // a CTA per eight atoms up to three of them per SM (126-64-64: 2000 atoms 25 against 45 us;
     // 4000 atoms 45 against 47)
     if (n <= 24 * sms && deep && cta <= kNetSmemMax) {
-        static size_t limit = 48 * 1024;
-        if (cta > limit) {
-            const cudaError_t e = cudaFuncSetAttribute(k_net_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cta);
-            if (e != cudaSuccess) return e;
-            limit = cta;
-        }
+        const cudaError_t e = allow_smem(k_net_cta, cta);
+        if (e != cudaSuccess) return e;
         return launch_pdl(&k_net_cta, dim3((n + kNetAtoms - 1) / kNetAtoms, count), dim3(kCtaThreads), cta, st, m);
     }
-    static size_t limit = 48 * 1024;
-    if (sm > limit) {
-        const cudaError_t e = cudaFuncSetAttribute(k_net_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        limit = sm;
-    }
+    const cudaError_t e = allow_smem(k_net_warp, sm);
+    if (e != cudaSuccess) return e;
     return launch_pdl(&k_net_warp, dim3((n + per_block - 1) / per_block, count), dim3(32 * wpc), sm, st, m, wf);
 }
 

@@ -52,6 +52,7 @@
 
 #include "net_tc.cuh"
 #include "pdl.cuh"
+#include "smem_limit.cuh"
 #include "tc_util.cuh"
 
 namespace nnapgb {
@@ -612,14 +613,8 @@ cudaError_t launch_net_tc(const NetArgs* a, const NetTC* const* tc, int nt, int*
     const bool two = L.staged && ntiles > 2 * sm_count && 2 * L.ncols <= 512 && L.smem + L.act <= kTcSmemTwo;
     void (*kern)(TcParams, TCLayout) = two ? k_net_tc<2, 2> : split == 2 ? k_net_tc<2, 1> : k_net_tc<4, 1>;
     const int smem = L.smem + (two ? L.act : 0);
-    static int limit[3] = {0, 0, 0};  // raised once per instantiation, before any graph capture
-    int& lim = limit[two ? 2 : split == 4];
-    if (smem > lim) {
-        const int most = two ? kTcSmemTwo : kTcSmemMax;
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        if (e != cudaSuccess) return e;
-        lim = most;
-    }
+    const cudaError_t e = allow_smem(kern, two ? kTcSmemTwo : kTcSmemMax);
+    if (e != cudaSuccess) return e;
     TcParams p;
     std::memset(&p, 0, sizeof p);
     p.perm = a[0].perm;

@@ -31,6 +31,7 @@
 
 #include <cuda_fp16.h>
 
+#include "smem_limit.cuh"
 #include "tc_util.cuh"
 
 namespace nnapgb {
@@ -349,13 +350,8 @@ __global__ void __launch_bounds__(32 * kFwdTcWarps, 4) k_sph_fwd_tc(DescArgs a) 
 template <int L, int NP, int N1>
 cudaError_t launch_sph_fwd_tc(const DescArgs& a, cudaStream_t st) {
     using S = SphTcShape<L, NP>;
-    static int lim = 0;
-    if (S::SMEM > lim) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(k_sph_fwd_tc<L, NP, N1>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
-        if (e != cudaSuccess) return e;
-        lim = S::SMEM;
-    }
+    const cudaError_t e = allow_smem(k_sph_fwd_tc<L, NP, N1>, S::SMEM);
+    if (e != cudaSuccess) return e;
     const int rounds = (a.nmax + kFwdTcWarps - 1) / kFwdTcWarps;
     const int grid = rounds < 4 * a.tc_sms ? rounds : 4 * a.tc_sms;
     return launch_pdl(&k_sph_fwd_tc<L, NP, N1>, dim3(grid), dim3(32 * kFwdTcWarps), (size_t)S::SMEM, st, a);

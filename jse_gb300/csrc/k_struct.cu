@@ -19,6 +19,7 @@
 #include "box_math.cuh"
 #include "common.cuh"
 #include "pdl.cuh"
+#include "smem_limit.cuh"
 
 namespace nnapgb {
 
@@ -744,11 +745,8 @@ static cudaError_t launch_nb(const StructDev* S, const int* sid, const double* x
                              const int* cell_of, const int* cell_start, const int* cell_atoms, int n, int warps,
                              const PairBufs& P, int* err, int* max_count, cudaStream_t st) {
     const size_t smem = warps * sizeof(NbWarp<SLOTS, NA>);
-    if (smem > 48 * 1024) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(k_neighbors<SLOTS, NA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_smem(k_neighbors<SLOTS, NA>, smem);
+    if (e != cudaSuccess) return e;
     const dim3 grid((unsigned)((n + warps * NA - 1) / (warps * NA))), block(32 * warps);
     // the kernels before have no shared memory: with many atoms each SM takes its split anew
     // (1048573 atoms 7159 -> 7078 us, 488206 5393 -> 5387, fewer the same)

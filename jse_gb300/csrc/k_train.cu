@@ -33,6 +33,7 @@
 #include "common.cuh"
 #include "desc.cuh"
 #include "sph_math.cuh"
+#include "smem_limit.cuh"
 #include "train.cuh"
 
 namespace nnapgb {
@@ -1048,13 +1049,8 @@ cudaError_t launch_radial_jvp(const JvpArgs& a, cudaStream_t st) {
     const int n = a.d.nmax;
     if (n <= 0) return cudaSuccess;
     const size_t sm = sizeof(float) * a.d.T * a.d.T * NP * Fuse<N1>::N1P;
-    static int lim = 0;
-    if ((int)sm > lim && sm > 48 * 1024) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(k_radial_jvp<NP, N1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        lim = (int)sm;
-    }
+    const cudaError_t e = allow_smem(k_radial_jvp<NP, N1>, sm);
+    if (e != cudaSuccess) return e;
     k_radial_jvp<NP, N1><<<(n + kJvpWarps - 1) / kJvpWarps, 32 * kJvpWarps, sm, st>>>(a);
     return cudaGetLastError();
 }
@@ -1064,13 +1060,8 @@ cudaError_t launch_sph_jvp_n(const JvpArgs& a, cudaStream_t st) {
     using S = JvpNShape<L, NP, N1>;
     const size_t sm = sizeof(float) * (((size_t)a.d.T * kFwdTypes * NP + 3) / 4 * 4 + (size_t)kJvpWarps * S::WARP_FLOATS);
     if (sm > 227 * 1024) return cudaErrorInvalidValue;
-    static int lim = 0;
-    if ((int)sm > lim) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(k_sph_jvp_n<L, NP, N1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        lim = (int)sm;
-    }
+    const cudaError_t e = allow_smem(k_sph_jvp_n<L, NP, N1>, sm);
+    if (e != cudaSuccess) return e;
     k_sph_jvp_n<L, NP, N1><<<(a.d.nmax + kJvpWarps - 1) / kJvpWarps, 32 * kJvpWarps, sm, st>>>(a);
     return cudaGetLastError();
 }
@@ -1083,13 +1074,8 @@ cudaError_t launch_sph_jvp(const JvpArgs& a, cudaStream_t st) {
     if (a.d.fwd_alpha && N1 < NP && a.d.T <= kFwdTypes) return launch_sph_jvp_n<L, NP, N1>(a, st);
     const size_t wf = ((size_t)a.d.T * a.d.T * NP * Fuse<N1>::N1P + 3) & ~(size_t)3;
     const size_t sm = sizeof(float) * (wf + (size_t)kJvpWarps * S::WARP_FLOATS);
-    static int lim = 0;
-    if ((int)sm > lim) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(k_sph_jvp<L, NP, N1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        lim = (int)sm;
-    }
+    const cudaError_t e = allow_smem(k_sph_jvp<L, NP, N1>, sm);
+    if (e != cudaSuccess) return e;
     k_sph_jvp<L, NP, N1><<<(n + kJvpWarps - 1) / kJvpWarps, 32 * kJvpWarps, sm, st>>>(a);
     return cudaGetLastError();
 }
@@ -1105,13 +1091,8 @@ cudaError_t launch_wgrad_t(const WgradArgs& g, cudaStream_t st) {
     const size_t wf = ((size_t)g.j.d.T * g.j.d.T * NP * Fuse<N1>::N1P + 3) & ~(size_t)3;
     const size_t sm = sizeof(float) * (wf + (size_t)kWgWarps * S::warp_floats(g.j.d.T));
     if (sm > 227 * 1024) return cudaErrorInvalidValue;
-    static int lim = 0;
-    if ((int)sm > lim) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(k_wgrad<L, NP, N1, SPH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        lim = (int)sm;
-    }
+    const cudaError_t e = allow_smem(k_wgrad<L, NP, N1, SPH>, sm);
+    if (e != cudaSuccess) return e;
     k_wgrad<L, NP, N1, SPH><<<(g.G + kWgWarps - 1) / kWgWarps, 32 * kWgWarps, sm, st>>>(g);
     return cudaGetLastError();
 }
@@ -1170,12 +1151,8 @@ cudaError_t launch_net_train(const NetTrainArgs* args, int count, cudaStream_t s
     while (wpc > 1 && (size_t)wpc * warp_floats * sizeof(float) > 200 * 1024) --wpc;
     const size_t sm = sizeof(float) * (size_t)warp_floats * wpc;
     if (sm > 227 * 1024) return cudaErrorInvalidValue;
-    static int lim = 0;
-    if ((int)sm > lim) {
-        const cudaError_t e = cudaFuncSetAttribute(k_net_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-        lim = (int)sm;
-    }
+    const cudaError_t e = allow_smem(k_net_train, sm);
+    if (e != cudaSuccess) return e;
     const int per_block = kTrainAtoms * wpc;
     k_net_train<<<dim3((n + per_block - 1) / per_block, count), 32 * wpc, sm, st>>>(m, warp_floats);
     return cudaGetLastError();

@@ -1,0 +1,103 @@
+"""The library's host path without a GPU: what it allocates, copies and launches.
+
+Child processes load a stand-in for the CUDA runtime (fake_cudart.cpp: host memory, kernels that do
+not run, two devices, the shared-memory limit of a launch as the runtime enforces it) ahead of
+libcudart.  Its values are zeros; the tests look at the calls."""
+import functools
+import os
+import shutil
+import subprocess
+import sys
+import tempfile
+import textwrap
+
+import pytest
+
+from tests.conftest import ROOT
+
+HEAD = """
+import ctypes as C, os, sys, threading, time
+import numpy as np
+F = C.CDLL(os.environ["FAKE_CUDART"])
+from jse_gb300 import nnap as J, workloads as W
+def log():
+    b = C.create_string_buffer(1 << 22)
+    assert F.fake_log(b, 1 << 22) < 1 << 22
+    return b.value.decode().splitlines()
+def launches(part):
+    return [l.split() for l in log() if l.startswith("launch") and part in l]
+def atoms(n, T=2, density=0.05):
+    return W.random_liquid(n, density, [1.0 / T] * T, 1.9, n)
+def sph(T, hidden, nmax=8, lmax=6, wtype="default"):
+    return W.write_model(["S%d" % t for t in range(T)],
+                         {"type": "spherical_chebyshev", "nmax": nmax, "lmax": lmax, "rcut": 6.0, "wtype": wtype}, hidden, 1)
+"""
+
+
+@functools.lru_cache(None)
+def _fake():
+    inc = [d for d in (os.environ.get("CUDA_HOME", ""), "/usr/local/cuda") if os.path.exists(os.path.join(d, "include", "cuda_runtime_api.h"))]
+    if not inc or not shutil.which("g++"):
+        pytest.skip("no CUDA headers or no g++")
+    from jse_gb300 import build, nnap
+    if not os.path.exists(nnap.LIB_PATH):
+        build.build()
+    out = os.path.join(tempfile.mkdtemp(), "libfakecudart.so")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I", os.path.join(inc[0], "include"),
+                    os.path.join(ROOT, "tests", "fake_cudart.cpp"), "-o", out, "-lpthread"], check=True)
+    return out
+
+
+def _child(code):
+    env = dict(os.environ, LD_PRELOAD=_fake(), FAKE_CUDART=_fake(), PYTHONPATH=ROOT)
+    r = subprocess.run([sys.executable, "-c", HEAD + textwrap.dedent(code)], env=env, cwd=ROOT, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
+
+
+def test_shared_memory_limits_of_a_second_device():
+    """Every launch beyond 48 KiB is allowed on each device that a handle is made for."""
+    _child("""
+    rng = np.random.default_rng(1)
+    deep = sph(3, [64, 64])
+    for device in (0, 1):
+        for model, T in ((deep, 3), (sph(1, [300, 100], 5), 1), (sph(8, [32], 5), 8), (sph(2, [20], 7, 5), 2)):
+            for precision in ("fp32", "mixed"):
+                with J.NNAP(model, precision=precision, device=device) as p:
+                    for n in (60, 4500, 50000):
+                        p.calForces(atoms(n, T))
+                    p.setTuning(4500, dict(p.tuning(4500), desc_fwd_warps=8, desc_bwd_warps=8, nb_warps=8))
+                    p.calForces(atoms(4500, T))
+                    p.calFp(atoms(60, T))
+        basis = {"type": "spherical_chebyshev", "nmax": 4, "lmax": 4, "rcut": 5.0, "wtype": "fuse", "fuse_size": 2}
+        fuse = W.write_model(["A", "B"], dict(basis, wtype="default"), [64, 64], 1)
+        for m in fuse["models"]:
+            m["basis"] = dict(basis, fuse_weight=rng.normal(0, 1, 4).tolist())
+        with J.NNAP(fuse, device=device) as p:
+            p.backwardEnergyForceBatch([atoms(40)], np.ones(40), np.ones((40, 3)), want_fp=True)
+    big = {int(l.split()[3]) for l in log() if l.startswith("launch") and int(l.split()[4]) > 48 * 1024}
+    assert big == {0, 1}, big
+    """)
+
+
+def test_shared_memory_limits_of_two_threads():
+    """A narrow network's call between another thread's raise of the limit and its launch."""
+    _child("""
+    s = atoms(4000, 3)
+    wide, narrow = J.NNAP(sph(3, [200, 200])), J.NNAP(sph(3, [64, 64]))
+    F.fake_pause(b"k_net_warp")
+    failed = []
+    def work():
+        try:
+            wide.calForces(s)
+        except Exception as e:
+            failed.append(e)
+    t = threading.Thread(target=work)
+    t.start()
+    while not F.fake_paused():
+        time.sleep(0.01)
+    narrow.calForces(s)
+    F.fake_resume()
+    t.join()
+    assert not failed, failed
+    """)
