@@ -23,6 +23,8 @@
 // one-nonzero-per-row fuse matrices runs on the tensor cores (k_sph_tc.cuh).
 #include <math_constants.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "pdl.cuh"
 #include "smem_limit.cuh"
@@ -590,6 +592,10 @@ __global__ void __launch_bounds__(32 * kDescMaxWarps, 2) k_sph_bwd(DescArgs a) {
 // batch (526k atoms, lmax 6) 2.55 -> 1.98 ms, 1M-atom glass (lmax 4) 3.19 -> 1.76 ms, 32000-atom
 // liquid 174 -> 139 us.  Two neighbours of one species per lane halve the reads but leave 11
 // warps per SM (165 registers): 2.45 ms on the batch.
+// Fuse rows that are not diagonal, and those of more than kFwdTypes species, are read in sparse
+// form as each atom needs them: its species' part is a few KB, the whole table 2 T^2 N1 kNz words,
+// which a CTA of four atoms copied to shared memory and kept (lmax 6, nmax 8, 20000 atoms: eight
+// species 322 -> 207 us, ten 600 -> 291, fifteen 1110 -> 527).
 template <int L, int NP, int N1>
 struct SphNShape {
     static constexpr int K = (L + 1) * (L + 1);
@@ -678,14 +684,8 @@ __global__ void __launch_bounds__(32 * kBwdWarps, LPA == 32 ? 5 : 6) k_sph_bwd_n
     float2* sCo = sN + S::NS;
     const bool diag = a.fwd_alpha != nullptr && T <= kFwdTypes;
     float* tab = smem + ((4 * S::NS + 3) & ~3);
-    const int ntab = diag ? 0 : T * T * N1 * kNz, nal = diag ? T * kFwdTypes * NP : 0;
-    int* sNp = reinterpret_cast<int*>(tab);
-    float* sNw = tab + ntab;
+    const int nal = diag ? T * kFwdTypes * NP : 0;
     float* sAl = tab;  // alpha[tc][tn][p] of fuse rows with their one nonzero in column p mod N1
-    for (int q = threadIdx.x; q < ntab; q += blockDim.x) {
-        sNp[q] = a.nz_p[q];
-        sNw[q] = a.nz_w[q];
-    }
     for (int q = threadIdx.x; q < nal; q += blockDim.x) sAl[q] = a.fwd_alpha[q];
     for (int s = threadIdx.x; s < S::NS; s += blockDim.x) {
         int l0, l1, m = 0;
@@ -708,7 +708,7 @@ __global__ void __launch_bounds__(32 * kBwdWarps, LPA == 32 ? 5 : 6) k_sph_bwd_n
     const int s0 = a.range[a.t0], s1 = a.range[a.t1];
     if (s0 + w0 >= s1) return;
     const bool act = s0 + w < s1;
-    float* sGh = tab + ((diag ? nal : 2 * ntab) + 3) / 4 * 4 + (size_t)(wl * APW + grp) * (T * S::GH + (diag ? 0 : (NP * S::K + 3) / 4 * 4));
+    float* sGh = tab + (nal + 3) / 4 * 4 + (size_t)(wl * APW + grp) * (T * S::GH + (diag ? 0 : (NP * S::K + 3) / 4 * 4));
     const int at = a.perm[act ? s0 + w : s0 + w0];
     const int tc = a.type[at] - 1;
     const int M = a.P.M, cnt = act ? min(a.P.count[at], M) : 0;
@@ -795,18 +795,22 @@ __global__ void __launch_bounds__(32 * kBwdWarps, LPA == 32 ? 5 : 6) k_sph_bwd_n
                     k0 = l * l + l + m;
                     k1 = l * l + l - m;
                 }
-                const int* np_ = sNp + (size_t)(tc * T + tn) * N1 * kNz;
-                const float* nw = sNw + (size_t)(tc * T + tn) * N1 * kNz;
+                // the sparse rows of (tc, tn), kNz = 4 words each
+                const int4* np4 = reinterpret_cast<const int4*>(a.nz_p) + (size_t)(tc * T + tn) * N1;
+                const float4* nw4 = reinterpret_cast<const float4*>(a.nz_w) + (size_t)(tc * T + tn) * N1;
                 float* out = sGh + tn * S::GH + s * S::RF;
 #pragma unroll
                 for (int n = 0; n < N1; ++n) {
                     float vx = 0.f, vy = 0.f;
+                    const int4 p4 = np4[n];
+                    const float4 w4 = nw4[n];
+                    const int pz[kNz] = {p4.x, p4.y, p4.z, p4.w};
+                    const float wz[kNz] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
                     for (int z = 0; z < kNz; ++z) {
-                        const int pp = np_[n * kNz + z];
-                        if (pp >= 0) {
-                            vx += nw[n * kNz + z] * scr[pp * S::K + k0];
-                            if (k1 >= 0) vy += nw[n * kNz + z] * scr[pp * S::K + k1];
+                        if (pz[z] >= 0) {
+                            vx += wz[z] * scr[pz[z] * S::K + k0];
+                            if (k1 >= 0) vy += wz[z] * scr[pz[z] * S::K + k1];
                         }
                     }
                     *reinterpret_cast<float2*>(out + 2 * n) = make_float2(vx, vy);
@@ -1146,11 +1150,24 @@ cudaError_t launch_sph_bwd_lanes(const DescArgs& a, cudaStream_t st) {
     using S = SphNShape<L, NP, N1>;
     constexpr int APW = 32 / LPA;
     const bool diag = a.fwd_alpha && a.T <= kFwdTypes;
-    const size_t fixed = (4 * (size_t)S::NS + 3) / 4 * 4 +
-                         ((diag ? (size_t)a.T * kFwdTypes * NP : (size_t)2 * a.T * a.T * N1 * kNz) + 3) / 4 * 4;
+    const size_t fixed = (4 * (size_t)S::NS + 3) / 4 * 4 + (diag ? (size_t)a.T * kFwdTypes * NP + 3 : 0) / 4 * 4;
+    auto bytes = [&](int w) { return sizeof(float) * (fixed + (size_t)w * S::warp_floats(a.T, APW, diag)); };
     int wpc = a.warps < kBwdWarps ? a.warps : kBwdWarps;
-    while (wpc > 1 && sizeof(float) * (fixed + (size_t)wpc * S::warp_floats(a.T, APW, diag)) > 227 * 1024) wpc >>= 1;
-    const size_t sm = sizeof(float) * (fixed + (size_t)wpc * S::warp_floats(a.T, APW, diag));
+    if (!diag) {
+        // many species: the CTA size that leaves the most warps on an SM by its shared memory
+        // (228 KB, 1 KB per CTA kept back) and registers
+        constexpr int reg_warps = LPA == 32 ? 21 : 25;
+        int best = 0;
+        for (int w = wpc; w >= 1; --w) {
+            const int ctas = std::min((int)(228 * 1024 / (bytes(w) + 1024)), reg_warps / w);
+            if (bytes(w) <= 227 * 1024 && w * ctas > best) {
+                best = w * ctas;
+                wpc = w;
+            }
+        }
+    }
+    while (wpc > 1 && bytes(wpc) > 227 * 1024) wpc >>= 1;
+    const size_t sm = bytes(wpc);
     if (sm > 227 * 1024) return cudaErrorInvalidValue;
     const int grid = (a.nmax + wpc * APW - 1) / (wpc * APW);
     const cudaError_t e = allow_smem(k_sph_bwd_n<L, NP, N1, LPA>, sm);

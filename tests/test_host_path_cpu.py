@@ -101,3 +101,18 @@ def test_shared_memory_limits_of_two_threads():
     t.join()
     assert not failed, failed
     """)
+
+
+def test_backward_warps_of_many_species():
+    """The backward's shared memory does not grow with the square of the species: eight warps or
+    more stay on an SM (228 KB, of which each CTA costs 1 KB more than it asks for)."""
+    _child("""
+    for T, lmax in ((4, 6), (10, 6), (12, 4), (15, 4)):
+        with J.NNAP(sph(T, [16], 8, lmax)) as p:
+            log()
+            p.calForces(atoms(600, T))
+            (l,) = launches("k_sph_bwd_n")
+            grid, threads, smem = int(l[1]), int(l[2]), int(l[4])
+            warps = threads // 32 * (228 * 1024 // (smem + 1024))
+            assert warps >= 8 and grid * threads // 32 >= 600, (T, lmax, l, warps)
+    """)
