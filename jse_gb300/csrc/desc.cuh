@@ -92,8 +92,11 @@ constexpr float kTcAlphaMax = 1024.f;  // largest |alpha| the tensor-core forwar
     X(6, 18, 9) X(4, 18, 9) X(4, 5, 5) X(2, 4, 4) X(2, 8, 4) X(2, 12, 4) X(3, 5, 4) X(2, 16, 4) \
     X(3, 10, 5) X(6, 9, 9) X(4, 9, 9) X(3, 8, 4) X(4, 10, 5)
 // Spherical shapes compiled for evaluation alone: the model format's defaults (nmax 5, lmax 6)
-// with several and with one species.
+// with several and with one species.  Their channel-space kernels serve up to kEvalTypes species:
+// the forward of 20000 atoms takes 108 us with six species and 165 with eight (680 with sixteen),
+// the any-shape one 138, 141 and 151.
 #define NNAP_SPH_EVAL_SHAPES(X) X(6, 12, 6) X(6, 6, 6)
+constexpr int kEvalTypes = 6;
 
 // Radial functions of a sub-basis: the NNAP Chebyshev basis or the NEP basis (radial_f /
 // radial_g in sph_math.cuh).

@@ -1253,7 +1253,11 @@ cudaError_t launch_descriptor(int kind, int basis, int lmax, int np, int n1, con
         constexpr int RB_ = kRbNNAP;
         NNAP_RADIAL_SHAPES(R_CASE)
         NNAP_SPH_SHAPES(S_CASE)
-        NNAP_SPH_EVAL_SHAPES(S_CASE)
+        // the evaluation shapes: the channel-space kernels keep the fuse matrices of all T^2 pairs
+        // in shared memory, so beyond kEvalTypes species the any-shape kernels are the faster
+        if (a.T <= kEvalTypes || (!fwd && a.nz_p && a.nz_w)) {
+            NNAP_SPH_EVAL_SHAPES(S_CASE)
+        }
     } else if (basis == kRbNEP) {
         constexpr int RB_ = kRbNEP;
         NEP_RADIAL_SHAPES(R_CASE)

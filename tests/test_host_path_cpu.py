@@ -116,3 +116,17 @@ def test_backward_warps_of_many_species():
             warps = threads // 32 * (228 * 1024 // (smem + 1024))
             assert warps >= 8 and grid * threads // 32 >= 600, (T, lmax, l, warps)
     """)
+
+
+def test_default_shape_of_many_species():
+    """The compiled forward of the default shape serves few species, the any-shape one many; the
+    radial-space backward serves them all."""
+    _child("""
+    for T, wtype in ((6, "default"), (7, "default"), (16, "default"), (6, "none"), (12, "none")):
+        with J.NNAP(sph(T, [16], 5, 6, wtype)) as p:
+            p.calForces(atoms(600, T))
+            names = [l.split()[5] for l in log() if l.startswith("launch")]
+            assert any("k_sph_bwd_n" in s for s in names), names
+            assert any("9k_sph_fwd" in s for s in names) == (T <= 6), (T, names)
+            assert any("k_sph_fwd_g" in s for s in names) == (T > 6), (T, names)
+    """)
