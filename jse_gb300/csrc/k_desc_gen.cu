@@ -27,7 +27,12 @@ cudaError_t launch_g(Kern kern, const DescArgs& a, size_t per_warp, int np, int 
     const cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return e;
     const int grid = (a.nmax + wpc - 1) / wpc;
-    return launch_pdl(kern, dim3(grid), dim3(32 * wpc), sm, st, a, np, n1);
+    // An SM that a kernel enters early keeps its predecessor's split between shared memory and L1;
+    // the forward comes after kernels without shared memory and needs tens of KB, the backward
+    // after a network with tens of KB and needs L1.  Launched after their predecessors: 33 radial
+    // functions, two species, 2000 atoms 201 -> 158 us a call, 3000 206 -> 171 (the forward alone
+    // 160 and 179); lmax 5, 500 atoms 149 -> 139; 60 atoms, 9000 and more the same.
+    return launch_after(kern, dim3(grid), dim3(32 * wpc), sm, st, a, np, n1);
 }
 
 template <int RB>

@@ -28,7 +28,8 @@ void note(const std::string& line) {
     std::lock_guard<std::mutex> g(mu);
     log_.push_back(line);
 }
-cudaError_t launch(const void* f, dim3 grid, dim3 block, size_t dyn) {
+// early: with the attribute that lets a kernel start before its predecessor ends
+cudaError_t launch(const void* f, dim3 grid, dim3 block, size_t dyn, bool early) {
     std::string name;
     size_t lim;
     {
@@ -40,7 +41,7 @@ cudaError_t launch(const void* f, dim3 grid, dim3 block, size_t dyn) {
     if (dyn > 48 * 1024 && dyn > lim) return cudaErrorInvalidValue;
     char line[160];
     std::snprintf(line, sizeof line, "launch %u %u %u %zu ", grid.x * grid.y, block.x, (unsigned)device, dyn);
-    note(line + name);
+    note(line + name + (early ? " early" : ""));
     return cudaSuccess;
 }
 cudaError_t give(void** p, size_t n) {
@@ -86,10 +87,14 @@ cudaError_t __cudaPopCallConfiguration(dim3* grid, dim3* block, size_t* dyn, voi
 }
 cudaError_t __cudaGetKernel(cudaKernel_t* k, const void* f) { *k = (cudaKernel_t)f; return cudaSuccess; }
 cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 grid, dim3 block, void**, size_t dyn, cudaStream_t) {
-    return launch((const void*)k, grid, block, dyn);
+    return launch((const void*)k, grid, block, dyn, false);
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) {
-    return launch(f, c->gridDim, c->blockDim, c->dynamicSmemBytes);
+    bool early = false;
+    for (unsigned q = 0; q < c->numAttrs; ++q)
+        early = early || (c->attrs[q].id == cudaLaunchAttributeProgrammaticStreamSerialization &&
+                          c->attrs[q].val.programmaticStreamSerializationAllowed);
+    return launch(f, c->gridDim, c->blockDim, c->dynamicSmemBytes, early);
 }
 cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
     if (a != cudaFuncAttributeMaxDynamicSharedMemorySize || v > 227 * 1024) return cudaErrorInvalidValue;

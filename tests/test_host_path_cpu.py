@@ -130,3 +130,18 @@ def test_default_shape_of_many_species():
             assert any("9k_sph_fwd" in s for s in names) == (T <= 6), (T, names)
             assert any("k_sph_fwd_g" in s for s in names) == (T > 6), (T, names)
     """)
+
+
+def test_any_shape_kernels_launch_after_their_predecessors():
+    """Early, they would run with the split of shared memory and L1 of the kernels before them."""
+    _child("""
+    for basis in ({"type": "chebyshev", "nmax": 15, "rcut": 4.0}, {"type": "spherical_chebyshev", "nmax": 6, "lmax": 5, "rcut": 5.0}):
+        model = W.write_model(["A", "B"], basis, [30], 1)
+        for precision in ("fp32", "mixed"):
+            with J.NNAP(model, precision=precision) as p:
+                log()
+                p.calForces(atoms(600))
+                l = [l for l in log() if l.startswith("launch")]
+                fwd, bwd = ([s for s in l if part in s] for part in ("fwd_g", "bwd_g"))
+                assert len(fwd) == len(bwd) == 1 and not fwd[0].endswith("early") and not bwd[0].endswith("early"), l
+    """)
