@@ -11,8 +11,8 @@
 //      species sort)
 //   -> descriptor forward (per run of species sharing a basis shape, per sub-basis)
 //   -> network per species -> descriptor backward -> k_gather -> k_reduce_chunks
-//   -> k_reduce_structs (left out where every structure is one chunk), for host calls of
-//   up to 2 MiB k_pack_results, then one host synchronisation (neighbour capacity, error bits).
+//   -> k_reduce_structs (left out where every structure is one chunk), for small
+//   host calls k_pack_results, then one host synchronisation (neighbour capacity, error bits).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1077,11 +1077,18 @@ void upload_inputs(nnap_handle* h, int n, const double* x, const int* type) {
     }
 }
 
-// A host call of at most kHostStage bytes in and out goes through pinned memory: one copy in, and
-// results written into mapped memory by the last kernel of the sequence, so the call has one
-// synchronisation and no pageable copies, whose fixed cost outweighs their bytes: 33 atoms 196 ->
-// 147 us, 4099 atoms 311 -> 259, 25000 atoms (1.5 MB) 559 -> 548.  Larger calls copy directly.
-constexpr size_t kHostStage = 2 << 20;
+// A small host call goes through pinned memory: one copy in, and results written into mapped
+// memory by the last kernel of the sequence, so the call has one synchronisation and no pageable
+// copies.  Each output so saved is worth 10 to 15 us (33 atoms, energies to virial: 139 -> 99 us a
+// call), each MB that is copied once more costs 30 to 50: forces alone break even at 0.4 MB in and
+// out (8000 atoms 164 either way, 14000 216 against 203 direct), energy and forces at 0.6 (8000
+// atoms 166 against 174, 14000 219 against 215), energy, energies, forces and virial at 1.1 (14000
+// 233 against 244, 20000 288 against 281; a program that then reads its results has them in its
+// cache, which is worth 20 us more there), all five at 1.0.  A caller whose memory is pinned saves
+// only launches and latencies: break even lies at a fifth of that (4000 atoms 131 against 128 us,
+// 25000 334 against 264).
+constexpr size_t kStageOutput = 320 << 10, kStageOutputPinned = 64 << 10;  // bytes per output
+constexpr int kStageOutputs = 4;                                          // and this many at most
 
 size_t host_bytes(const Batch& B, int flags) {
     const size_t n = B.natoms, S = B.nstruct;
@@ -1092,6 +1099,23 @@ size_t host_bytes(const Batch& B, int flags) {
     if (flags & NNAP_WANT_VIRIAL) d += 9 * S;
     if (flags & NNAP_WANT_VIRIALS) d += 9 * n;
     return sizeof(double) * d + (3 * sizeof(double) + sizeof(int)) * n;
+}
+
+bool stage_host_call(const Batch& B, int flags, const double* x) {
+    if (!B.natoms || !flags) return false;
+    size_t outs = 0;
+    for (int bit : {NNAP_WANT_ENERGY, NNAP_WANT_ENERGIES, NNAP_WANT_FORCES, NNAP_WANT_VIRIAL, NNAP_WANT_VIRIALS})
+        outs += (flags & bit) != 0;
+    outs = std::min<size_t>(outs, kStageOutputs);
+    const size_t bytes = host_bytes(B, flags);
+    if (bytes <= outs * kStageOutputPinned) return true;
+    if (bytes > outs * kStageOutput) return false;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, x) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return at.type == cudaMemoryTypeUnregistered;
 }
 
 void compute_staged(nnap_handle* h, const Batch& B, const double* x, const int* type, int flags, const Outputs& o) {
@@ -1346,7 +1370,7 @@ int nnap_compute_batch(nnap_handle* h, int nstruct, const int* natoms, const dou
         h->launches = 0;
         const Batch& B = plan_batch(h, nstruct, natoms, box_kind, boxes);
         if (B.natoms && (!x || !type)) throw ApiFail(NNAP_ERR_ARG, "positions or types are NULL");
-        if (B.natoms && flags && host_bytes(B, flags) <= kHostStage) {
+        if (stage_host_call(B, flags, x)) {
             compute_staged(h, B, x, type, flags, o);
             return NNAP_OK;
         }

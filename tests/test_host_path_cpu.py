@@ -145,3 +145,35 @@ def test_any_shape_kernels_launch_after_their_predecessors():
                 fwd, bwd = ([s for s in l if part in s] for part in ("fwd_g", "bwd_g"))
                 assert len(fwd) == len(bwd) == 1 and not fwd[0].endswith("early") and not bwd[0].endswith("early"), l
     """)
+
+
+def test_staging_by_size_and_memory():
+    """Small host calls are staged; larger ones, and sooner those whose memory is pinned, copy
+    straight between the caller's arrays and the device."""
+    _child("""
+    model = W.write_model(["A", "B"], {"type": "chebyshev", "nmax": 3, "rcut": 4.0}, [4], 1)
+    cudart = F
+    def host(a, pinned):
+        if not pinned:
+            return np.array(a)
+        p = C.c_void_p()
+        assert cudart.cudaMallocHost(C.byref(p), C.c_size_t(a.nbytes)) == 0
+        b = np.frombuffer((C.c_char * a.nbytes).from_address(p.value), dtype=a.dtype).reshape(a.shape)
+        b[...] = a
+        return b
+    for n, pinned, staged in ((30, False, True), (30, True, True), (4000, False, True), (4000, True, False), (8000, False, True),
+                              (16000, False, False), (16000, True, False)):
+        s = atoms(n)
+        x, t, e, f = (host(a, pinned) for a in (s.x, s.types, np.zeros(1), np.zeros((n, 3))))
+        with J.NNAP(model) as p:
+            box = np.ascontiguousarray(s.box.reshape(9))
+            for _ in range(2):
+                log()
+                p._check(p._L.nnap_compute(p._handle(), n, J._dptr(x), J._iptr(t), s.box_kind, J._dptr(box), 5, J._dptr(e), None,
+                                           J._dptr(f), None, None))
+                calls = log()
+                ends = {int(v) for l in calls if l.startswith("copy") for v in l.split()[3:]}
+                assert any("k_pack_results" in l for l in calls) == staged, (n, pinned, calls)
+                for a in (x, f):
+                    assert (a.ctypes.data in ends) == (not staged), (n, pinned, calls)
+    """)
