@@ -1118,6 +1118,13 @@ bool stage_host_call(const Batch& B, int flags, const double* x) {
     return at.type == cudaMemoryTypeUnregistered;
 }
 
+// Staging grows by doubling: a caller whose atom count rises step by step allocates now and then.
+size_t stage_room(size_t bytes) {
+    size_t room = 4096;
+    while (room < bytes) room *= 2;
+    return room;
+}
+
 void compute_staged(nnap_handle* h, const Batch& B, const double* x, const int* type, int flags, const Outputs& o) {
     const size_t n = B.natoms, xb = 3 * sizeof(double) * n, tb = sizeof(int) * n;
     const size_t len[5] = {(size_t)B.nstruct, n, 3 * n, 9 * (size_t)B.nstruct, 9 * n};
@@ -1128,9 +1135,9 @@ void compute_staged(nnap_handle* h, const Batch& B, const double* x, const int* 
         h->pack_off[k] = flags & bit[k] ? (int)total : -1;
         if (flags & bit[k]) total += len[k];
     }
-    char* in = static_cast<char*>(h->pin_in.ensure(xb + tb));
-    const double* out = static_cast<const double*>(h->pin_out.ensure(sizeof(double) * std::max<size_t>(total, 1)));
-    h->dev_in.ensure(xb + tb);
+    char* in = static_cast<char*>(h->pin_in.ensure(stage_room(xb + tb)));
+    const double* out = static_cast<const double*>(h->pin_out.ensure(stage_room(sizeof(double) * total)));
+    h->dev_in.ensure(stage_room(xb + tb));
     std::memcpy(in, x, xb);
     std::memcpy(in + xb, type, tb);
     CK(cudaMemcpyAsync(h->dev_in.p, in, xb + tb, cudaMemcpyHostToDevice, h->stream));

@@ -177,3 +177,19 @@ def test_staging_by_size_and_memory():
                 for a in (x, f):
                     assert (a.ctypes.data in ends) == (not staged), (n, pinned, calls)
     """)
+
+
+def test_staging_of_a_growing_structure():
+    """Insertion moves: an atom more per call, and few allocations of pinned memory for all of them."""
+    _child("""
+    model = W.write_model(["A", "B"], {"type": "chebyshev", "nmax": 3, "rcut": 4.0}, [4], 1)
+    s = atoms(400)
+    with J.NNAP(model) as p:
+        p.calForces(W.Structure(s.x[:100], s.types[:100], s.box, s.box_kind))
+        log()
+        for n in range(101, 401):
+            p.calForces(W.Structure(s.x[:n], s.types[:n], s.box, s.box_kind))
+        calls = log()
+        assert sum("k_pack_results" in l for l in calls) == 300
+        assert sum(l.startswith("host_alloc") for l in calls) <= 6, [l for l in calls if l.startswith("host_")]
+    """)
