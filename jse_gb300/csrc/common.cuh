@@ -48,6 +48,7 @@ __host__ __device__ inline uint64_t pair_key(int j, uint32_t img) { return ((uin
 
 // Device buffers of one evaluation (all owned by the handle; see nnap_api.cu).
 constexpr int kLmpSumThreads = 256;  // threads of the LAMMPS global-virial sum
+constexpr int kLmpLanes = 8;         // lanes per atom of the LAMMPS gather
 
 struct PairBufs {
     int M;                 // neighbour capacity per atom (row stride)

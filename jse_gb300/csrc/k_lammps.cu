@@ -107,8 +107,6 @@ __global__ void k_lmp_fill(PairBufs P, int inum, const int* __restrict__ tstart,
 // kLmpLanes-th entry as float-float; a fixed butterfly adds the lanes; FP64 output.  The time is
 // the chain of scattered loads: one thread per atom 64 us for 8000 atoms and 9000 ghosts, eight
 // lanes 17 us.
-constexpr int kLmpLanes = 8;
-
 __device__ __forceinline__ void lmp_merge(float& h, float& l, unsigned mask, int off) {
     const float oh = __shfl_xor_sync(mask, h, off), ol = __shfl_xor_sync(mask, l, off);
     float s, e;

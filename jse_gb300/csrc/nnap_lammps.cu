@@ -168,8 +168,8 @@ int compute_lammps(nnap_handle* h, int nlflag, int inum, int nall, const int* il
         }
         k_sort_cells<<<(unsigned)(((size_t)nall * 32 + 255) / 256), 256, 0, st>>>(h->lmp_tstart.p, nall,
                                                                                   h->lmp_tlist.p);
-        k_lmp_gather<<<(unsigned)(((size_t)nall * 8 + 127) / 128), 128, 0, st>>>(pair_bufs(h), nall, h->lmp_rowof.p, h->lmp_tstart.p,
-                                                         h->lmp_tlist.p, h->lmp_forces.p, h->lmp_virials.p);
+        k_lmp_gather<<<(unsigned)(((size_t)nall * kLmpLanes + 127) / 128), 128, 0, st>>>(
+            pair_bufs(h), nall, h->lmp_rowof.p, h->lmp_tstart.p, h->lmp_tlist.p, h->lmp_forces.p, h->lmp_virials.p);
         h->launches += 3;
         CK(cudaGetLastError());
         // results back (pinned) and into LAMMPS's accumulators; a global virial alone is
