@@ -1120,9 +1120,23 @@ bool stage_host_call(const Batch& B, int flags, const double* x) {
 
 // Staging grows by doubling: a caller whose atom count rises step by step allocates now and then.
 size_t stage_room(size_t bytes) {
+    if (bytes > kStageOutputs * kStageOutput) return bytes;  // not staged
     size_t room = 4096;
     while (room < bytes) room *= 2;
     return room;
+}
+
+// Device inputs of a host call: one array, positions then types, staged or not.  A captured
+// sequence names its inputs, so calls of one layout that take turns between the two (forces, then
+// the energy alone) replay the same one.
+struct CallInputs {
+    double* x;
+    int* type;
+};
+
+CallInputs call_inputs(nnap_handle* h, size_t n) {
+    h->dev_in.ensure(stage_room((3 * sizeof(double) + sizeof(int)) * n));
+    return {reinterpret_cast<double*>(h->dev_in.p), reinterpret_cast<int*>(h->dev_in.p + 3 * sizeof(double) * n)};
 }
 
 void compute_staged(nnap_handle* h, const Batch& B, const double* x, const int* type, int flags, const Outputs& o) {
@@ -1137,16 +1151,16 @@ void compute_staged(nnap_handle* h, const Batch& B, const double* x, const int* 
     }
     char* in = static_cast<char*>(h->pin_in.ensure(stage_room(xb + tb)));
     const double* out = static_cast<const double*>(h->pin_out.ensure(stage_room(sizeof(double) * total)));
-    h->dev_in.ensure(stage_room(xb + tb));
+    const CallInputs d = call_inputs(h, n);
     std::memcpy(in, x, xb);
     std::memcpy(in + xb, type, tb);
-    CK(cudaMemcpyAsync(h->dev_in.p, in, xb + tb, cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemcpyAsync(d.x, in, xb + tb, cudaMemcpyHostToDevice, h->stream));
     struct Packing {
         int& f;
         ~Packing() { f = 0; }
     } packing{h->pack_flags};
     h->pack_flags = flags;
-    evaluate(h, B, reinterpret_cast<const double*>(h->dev_in.p), reinterpret_cast<const int*>(h->dev_in.p + xb), false);
+    evaluate(h, B, d.x, d.type, false);
     for (int k = 0; k < 5; ++k)
         if (flags & bit[k]) std::memcpy(dst[k], out + h->pack_off[k], sizeof(double) * len[k]);
 }
@@ -1381,8 +1395,12 @@ int nnap_compute_batch(nnap_handle* h, int nstruct, const int* natoms, const dou
             compute_staged(h, B, x, type, flags, o);
             return NNAP_OK;
         }
-        upload_inputs(h, B.natoms, x, type);
-        evaluate(h, B, h->x.p, h->type.p, false);
+        const CallInputs d = call_inputs(h, B.natoms);
+        if (B.natoms) {
+            CK(cudaMemcpyAsync(d.x, x, 3 * sizeof(double) * B.natoms, cudaMemcpyHostToDevice, h->stream));
+            CK(cudaMemcpyAsync(d.type, type, sizeof(int) * B.natoms, cudaMemcpyHostToDevice, h->stream));
+        }
+        evaluate(h, B, d.x, d.type, false);
         copy_out(h, B, flags, o, cudaMemcpyDeviceToHost);
         CK(cudaStreamSynchronize(h->stream));
         return NNAP_OK;

@@ -193,3 +193,22 @@ def test_staging_of_a_growing_structure():
         assert sum("k_pack_results" in l for l in calls) == 300
         assert sum(l.startswith("host_alloc") for l in calls) <= 6, [l for l in calls if l.startswith("host_")]
     """)
+
+
+def test_calls_that_alternate_share_a_captured_sequence():
+    """Forces (copied directly at this size) and the energy alone (staged) in turn: the launch
+    sequence of the layout is captured once."""
+    _child("""
+    model = W.write_model(["A", "B"], {"type": "chebyshev", "nmax": 3, "rcut": 4.0}, [4], 1)
+    s = atoms(8000)
+    box = np.ascontiguousarray(s.box.reshape(9))
+    e, f = np.zeros(1), np.zeros((8000, 3))
+    with J.NNAP(model) as p:
+        log()
+        for k in range(12):
+            p._check(p._L.nnap_compute(p._handle(), 8000, J._dptr(s.x), J._iptr(s.types), s.box_kind, J._dptr(box), 4 if k % 2 else 1,
+                                       J._dptr(e), None, J._dptr(f), None, None))
+        calls = log()
+        assert sum("k_pack_results" in l for l in calls) == 6, "the sizes no longer straddle the limit"
+        assert calls.count("capture") == 1, calls.count("capture")
+    """)
