@@ -165,11 +165,12 @@ def load_peaks():
 def load_traffic():
     """DRAM bytes per atom of a stage's dominant kernel, from one ncu capture
     (dram__bytes_read.sum + dram__bytes_write.sum of one launch divided by its atoms):
-    liquid32k / descriptors_bwd is k_sph_bwd_n<6,18,9> on the 32000-atom liquid, 159.2 MB
-    read + 16.9 MB written (profiles/k_sph_liquid32k.md); batch1024 / descriptors_bwd is the
-    same kernel over the 1024-structure batch, 2626.6 MB read + 443.2 MB written for 526124
-    atoms (profiles/batch1024_launches_and_top_kernels.md)."""
-    return {"liquid32k/descriptors_bwd": (159.2e6 + 16.9e6) / 32000,
+    liquid32k / descriptors_bwd is k_sph_bwd_n<6,18,9> on the 32000-atom liquid, 161.0 MB
+    read + 17.4 MB written (profiles/counters_main_kernels.md); batch1024 / descriptors_bwd is
+    the kernel over the 1024-structure batch, 2626.6 MB read + 443.2 MB written for 526124
+    atoms, captured on its earlier form, which reads and writes the same arrays
+    (profiles/batch1024_launches_and_top_kernels.md)."""
+    return {"liquid32k/descriptors_bwd": (161.0e6 + 17.4e6) / 32000,
             "batch1024/descriptors_bwd": (2626.569e6 + 443.240e6) / 526124}
 
 

@@ -135,11 +135,12 @@ struct Run {
     std::vector<int> fp_off;
     std::vector<DevBuf<float>> W;  // per sub: [T][T][NP][N1]
     // per sub: sparse form of W ([T][T][N1][kNz] rows and weights), empty when a column
-    // has more than kNz nonzero rows or N1 >= NP (the backward then stays in NP space)
+    // has more than kNz nonzero rows, N1 > NP, or N1 == NP with compact rows (the backward then
+    // stays in NP space)
     std::vector<DevBuf<int>> nzp;
     std::vector<DevBuf<float>> nzw;
     // per sub: alpha[tc][tn][p] of the radial-space forward ([T][kFwdTypes][NP]), empty
-    // unless every row p of W has its only nonzero in column p mod N1, N1 < NP, T <= kFwdTypes
+    // unless every row p of W has its only nonzero in column p mod N1, N1 <= NP, T <= kFwdTypes
     std::vector<DevBuf<float>> falpha;
     // per sub: the forward may run on the tensor cores (falpha present, every |alpha| at
     // most kTcAlphaMax); used in mixed precision

@@ -160,7 +160,8 @@ struct SphShape {
 };
 
 // Power spectrum of one atom from A [NP][K] in shared memory, a thread per channel: its K reads
-// walk the row with the loop over l unrolled (rows of odd length: no bank conflicts).
+// walk the row with the loop over l unrolled.  Rows of odd length (even L) meet no bank conflicts;
+// those of odd L do, on NP K of the reads.
 template <int L, int NP>
 __device__ __forceinline__ void power_rows(const float* A, int nl2, int sl, float* __restrict__ out, int t, int nt) {
     constexpr int K = (L + 1) * (L + 1);
@@ -295,7 +296,8 @@ struct SphFNShape {
 };
 
 // 1M-atom glass (lmax 4) 2.51 -> 2.04 ms with the angle-free harmonics and the spectrum by a
-// thread per channel (1500 warp instructions per atom; the shared-memory path is 75 % busy).
+// thread per channel (1513 warp instructions per atom of 40 neighbours; the shared-memory path is
+// 77 % busy: 131072 atoms).
 template <int L, int NP, int N1>
 __global__ void __launch_bounds__(32 * kDescMaxWarps) k_sph_fwd_n(DescArgs a) {
     using S = SphFNShape<L, NP, N1>;
@@ -587,9 +589,9 @@ __global__ void __launch_bounds__(32 * kDescMaxWarps, 2) k_sph_bwd(DescArgs a) {
 // side as float2 in shared memory, so one paired FMA serves both.
 //
 // Every lane reads N1 (L+1)^2 floats of Gh for each neighbour, and shared memory returns 128
-// bytes per cycle and SM: that path is 86 % busy (the FMA pipe 52 %), against the angle-based
+// bytes per cycle and SM: that path is 84 % busy (the FMA pipe 52 %; 32000 atoms), against the angle-based
 // walk with stored Legendre columns before, which issued twice the instructions.  1024-structure
-// batch (526k atoms, lmax 6) 2.55 -> 1.98 ms, 1M-atom glass (lmax 4) 3.19 -> 1.76 ms, 32000-atom
+// batch (488206 atoms, lmax 6) 2.55 -> 1.98 ms, 1M-atom glass (lmax 4) 3.19 -> 1.76 ms, 32000-atom
 // liquid 174 -> 139 us.  Two neighbours of one species per lane halve the reads but leave 11
 // warps per SM (165 registers): 2.45 ms on the batch.
 // Fuse rows that are not diagonal, and those of more than kFwdTypes species, are read in sparse

@@ -471,8 +471,10 @@ cudaError_t launch_net_fp32(const NetArgs* args, int count, int sms, cudaStream_
         if (e != cudaSuccess) return e;
         return launch_pdl(&k_net_fp32, dim3((n + per_block - 1) / per_block), dim3(32 * wpc), sm, st, args[0], wf);
     }
-    // a CTA per eight atoms up to three of them per SM (126-64-64: 2000 atoms 25 against 45 us;
-    // 4000 atoms 45 against 47)
+    // a CTA per eight atoms up to three of them per SM.  The CTA form takes a step with each CTA that
+    // an SM gets, the warp form is flat until SMs fill: up to 2400 atoms 24 against 45 us for
+    // 126-64-64 and 22 against 28 for 84-32-32, from there to this limit (3648 atoms) 43 against 45
+    // and 37 against 29, beyond it (5000) 58 against 49 and 51 against 31
     if (n <= 24 * sms && deep && cta <= kNetSmemMax) {
         const cudaError_t e = allow_smem(k_net_cta, cta);
         if (e != cudaSuccess) return e;

@@ -59,9 +59,10 @@ struct SphTcShape {
     // at least 46 KB, so that at most four CTAs (4 x 128 TMEM columns) share an SM
     static constexpr int SMEM = AL_BYTES + OPS > 47104 ? AL_BYTES + OPS : 47104;
     // lmax 6 or 7, where the tile's 64 rows are mostly in use, and 16 or more channels.  Each MMA
-    // truncates its FP32 accumulation, so descriptors are within 9e-7 of 64 bits where the FP32
-    // pipe's are within 3e-7: smaller shapes, which gain less, stay there (lmax 4 with two atoms
-    // per tile: 1.65 against 2.05 ms on the 1M-atom glass)
+    // truncates its FP32 accumulation: descriptors of the liquid are 2.4e-7 (rms; 2.5e-6 at most)
+    // of a column's largest off 64 bits, the FP32 pipe's 1.5e-7 (2.0e-6).  Smaller shapes, which
+    // gain less, stay there (lmax 4 with two atoms per tile: 1.65 against 2.05 ms on the 1M-atom
+    // glass)
     static constexpr bool fits = KM >= 49 && KM <= 64 && NP >= 16 && NPN <= 32;
 };
 
@@ -90,7 +91,7 @@ __device__ __forceinline__ void split_f16x8(const float* v, uint4& hi, uint4& lo
     lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
-// Bound: instruction issue (1716 warp instructions per atom of 54 neighbours, 53 % of the slots;
+// Bound: instruction issue (1816 warp instructions per atom of 54 neighbours, 52 % of the slots;
 // the operand splits and stores are a third).  Angle-free harmonics, a read-back by both halves
 // of each warp, the spectrum by a thread per channel and the next atom's loads ahead of their
 // use: 1024-structure batch 2.00 -> 1.32 ms, 32000-atom liquid 139 -> 97 us.

@@ -190,9 +190,9 @@ __global__ void k_sort_cells(const int* __restrict__ cell_start, int ncells, int
 // Candidate positions are read from the cell-ordered copies xfc / xloc (k_cell_order), so
 // a lane's atom index and position loads are independent and a cell's candidates are
 // contiguous in memory.
-// Bound: instruction issue and its dependences (1145 warp instructions per atom at 24 warps per
-// SM, 53 % of the issue slots with 8 atoms per warp; one atom per warp, which set up its cells and looked up the cell
-// of each candidate for itself, took 2068 at 75 %).  Neighbour stage of the batch of 1024
+// Bound: instruction issue and its dependences (131072 atoms, 8 per warp: 1106 warp instructions
+// per atom, 63 % of the issue slots at 20 warps per SM; one atom per warp, which set up its cells
+// and looked up the cell of each candidate for itself, took 2068 at 75 % on the batch).  Neighbour stage of the batch of 1024
 // structures 1.78 -> 1.40 ms, of the 1M-atom glass 3.05 -> 2.33 ms.
 constexpr int kNbMaxWarps = 8;  // warps per CTA are a launch parameter (2, 4 or 8)
 constexpr int kNbAtoms = 8;     // most atoms per warp

@@ -95,7 +95,8 @@ cudaError_t launch_jvp(int kind, int lmax, int np, int n1, const JvpArgs& a, cud
 cudaError_t launch_net_train(const NetTrainArgs* a, int count, cudaStream_t st);
 cudaError_t launch_train_reduce(const ReduceArgs& a, cudaStream_t st);
 cudaError_t launch_wgrad(int kind, int lmax, int np, int n1, const WgradArgs& a, cudaStream_t st);
-// out[e] = sum over w < G of partial[w * per + e] (FP64, in w order), e < per.
+// out[e] = sum over w < G of partial[w * per + e] (FP64, in a fixed order: 32 interleaved sums,
+// added in order), e < per.
 cudaError_t launch_wgrad_final(const float* partial, int G, int per, double* out, cudaStream_t st);
 
 }  // namespace nnapgb
