@@ -238,7 +238,8 @@ int nnap_set_graphs(nnap_handle* h, int on);
  * threads per row of the tensor-core network) and keeps the fastest; later evaluations
  * of the bucket reuse them.  Off by default; untuned buckets use 4, 4, 4, 128, 4.  The
  * backward of the compiled spherical shapes runs at most 4 warps (8 means 4), and the network
- * 2 threads per row where a CTA has two tiles in flight. */
+ * 2 threads per row where a CTA has two tiles in flight; what would run the same is
+ * not timed. */
 int nnap_set_autotune(nnap_handle* h, int on);
 /* Shapes used for natoms atoms: [descriptor forward warps, descriptor backward warps,
  * neighbour warps, gather threads, network threads per row]; *tuned = 1 when the

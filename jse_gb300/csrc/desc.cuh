@@ -119,6 +119,8 @@ cudaError_t launch_subrows(const PairBufs& P, int n, float rc, float4* sdx, int*
 // desc_supported: that, or the any-shape kernels of k_desc_gen.cu fit in shared memory.
 bool desc_compiled(int kind, int basis, int lmax, int np, int n1);
 bool desc_supported(int kind, int basis, int lmax, int np, int n1);
+// Most warps per CTA that the backward of a sub-basis runs; sparse: DescArgs::nz_p is given.
+int desc_bwd_max_warps(int kind, int basis, int lmax, int np, int n1, bool sparse);
 // Specialised instance when there is one, else the any-shape kernels.
 cudaError_t launch_descriptor(int kind, int basis, int lmax, int np, int n1, const DescArgs& a, bool fwd,
                               cudaStream_t st);

@@ -1246,6 +1246,16 @@ bool desc_compiled(int kind, int basis, int lmax, int np, int n1) {
     return false;
 }
 
+int desc_bwd_max_warps(int kind, int basis, int lmax, int np, int n1, bool sparse) {
+    if (basis == kRbNNAP && sparse) {
+#define S_CASE(L_, P_, N_) if (kind == 1 && lmax == L_ && np == P_ && n1 == N_ && N_ <= P_) return kBwdWarps;
+        NNAP_SPH_SHAPES(S_CASE)
+        NNAP_SPH_EVAL_SHAPES(S_CASE)
+#undef S_CASE
+    }
+    return kDescMaxWarps;
+}
+
 cudaError_t launch_descriptor(int kind, int basis, int lmax, int np, int n1, const DescArgs& a, bool fwd,
                               cudaStream_t st) {
 #define R_CASE(P_, N_) if (kind == 0 && np == P_ && n1 == N_) return launch_radial<P_, N_, RB_>(a, fwd, st);

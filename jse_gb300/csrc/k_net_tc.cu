@@ -594,6 +594,17 @@ void net_tc_release(NetTC& tc) {
     tc.ready = false;
 }
 
+static int max_tiles(int n, int nt) { return (n + 127) / 128 + nt; }  // over all species of a launch
+
+// Two tiles in flight once every SM has more than two: 40000 atoms (90-64-64-1) 36 us against
+// 41 with one, 200000 94 against 116; (126-64-64-1) 32000 atoms 36.5 against 35.8, 50000 51
+// against 48, 70000 57 against 60, 200000 121 against 139.  Both groups of a CTA need the
+// operand buffer (226 KiB in all) and TMEM columns (512).
+bool net_tc_two_tiles(const NetTC& tc, int n, int nt, int sm_count) {
+    const TCLayout& L = tc.L;
+    return L.staged && max_tiles(n, nt) > 2 * sm_count && 2 * L.ncols <= 512 && L.smem + L.act <= kTcSmemTwo;
+}
+
 cudaError_t launch_net_tc(const NetArgs* a, const NetTC* const* tc, int nt, int* err, int sm_count, int split,
                           cudaStream_t st) {
     if (nt < 1 || nt > kMaxTypes) return cudaErrorInvalidValue;
@@ -605,12 +616,8 @@ cudaError_t launch_net_tc(const NetArgs* a, const NetTC* const* tc, int nt, int*
     if (n <= 0) return cudaSuccess;
     const TCLayout& L = tc[0]->L;
     if (split != 2 && split != 4) return cudaErrorInvalidValue;
-    const int ntiles = (n + 127) / 128 + nt;  // upper bound of the tiles over all species
-    // Two tiles in flight once every SM has more than two: 40000 atoms (90-64-64-1) 36 us against
-    // 41 with one, 200000 94 against 116; (126-64-64-1) 32000 atoms 36.5 against 35.8, 50000 51
-    // against 48, 70000 57 against 60, 200000 121 against 139.  Both groups of a CTA need the
-    // operand buffer (226 KiB in all) and TMEM columns (512).
-    const bool two = L.staged && ntiles > 2 * sm_count && 2 * L.ncols <= 512 && L.smem + L.act <= kTcSmemTwo;
+    const int ntiles = max_tiles(n, nt);
+    const bool two = net_tc_two_tiles(*tc[0], n, nt, sm_count);
     void (*kern)(TcParams, TCLayout) = two ? k_net_tc<2, 2> : split == 2 ? k_net_tc<2, 1> : k_net_tc<4, 1>;
     const int smem = L.smem + (two ? L.act : 0);
     const cudaError_t e = allow_smem(kern, two ? kTcSmemTwo : kTcSmemMax);

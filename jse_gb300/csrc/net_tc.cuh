@@ -48,6 +48,8 @@ struct NetTC {
 // with the FP32 kernel).
 bool net_tc_prepare(const Species& sp, NetTC& tc, std::string& why);
 void net_tc_release(NetTC& tc);
+// Whether a launch over nt species and n atoms keeps two tiles in flight per CTA.
+bool net_tc_two_tiles(const NetTC& tc, int n, int nt, int sm_count);
 // One launch over nt consecutive species a[k].t = a[0].t + k, all with the same layout.
 // err receives ERRBIT_TIMEOUT if a bounded wait on the tensor cores gave up.
 // split: threads per tile row in the epilogues (2 or 4) where a CTA has one tile in flight; two

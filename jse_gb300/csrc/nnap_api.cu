@@ -928,11 +928,24 @@ Tuning tune_launches(nnap_handle* h, const Batch& B, const double* d_x, const in
         int stage;
         std::vector<int> cand;
     };
+    // only shapes that differ: the warps that some backward kernel runs, and the network's threads
+    // per row where some launch has one tile in flight
+    int bwd_warps = 0;
+    for (auto& r : h->runs)
+        for (size_t k = 0; k < r.subs.size(); ++k) {
+            const SubShape& s = r.subs[k];
+            bwd_warps = std::max(bwd_warps, desc_bwd_max_warps(s.kind, s.basis, s.lmax, s.np, s.n1, r.nzp[k].p != nullptr));
+        }
+    std::vector<int> bwd;
+    for (int w : {2, 4, 8})
+        if (w <= bwd_warps) bwd.push_back(w);
+    bool split = false;
+    for (auto& nd : h->nets) split = split || (h->net_tc && nd.tc.ready && !net_tc_two_tiles(nd.tc, B.natoms, 1, h->sm_count));
     std::vector<Param> params = {{&Tuning::nb_warps, 0, {2, 4, 8}},
                                  {&Tuning::desc_fwd_warps, 1, {2, 4, 8}},
-                                 {&Tuning::desc_bwd_warps, 3, {2, 4, 8}},
+                                 {&Tuning::desc_bwd_warps, 3, bwd},
                                  {&Tuning::gather_block, 4, {64, 128, 256}}};
-    if (h->net_tc) params.push_back({&Tuning::net_split, 2, {2, 4}});
+    if (split) params.push_back({&Tuning::net_split, 2, {2, 4}});
     try {
         for (auto& p : params) {
             int bv = best.*(p.field);

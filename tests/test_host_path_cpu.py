@@ -212,3 +212,21 @@ def test_calls_that_alternate_share_a_captured_sequence():
         assert sum("k_pack_results" in l for l in calls) == 6, "the sizes no longer straddle the limit"
         assert calls.count("capture") == 1, calls.count("capture")
     """)
+
+
+def test_autotuner_times_shapes_that_differ():
+    """Two runs and a warm-up per candidate: the backward of compiled shapes runs at most four warps,
+    the network has no choice of threads per row with two tiles in flight."""
+    _child("""
+    for model, n, precision, shapes in ((sph(2, [16], 5), 600, "fp32", 11), (sph(2, [16], 4, 5), 600, "fp32", 12),
+                                        (sph(2, [16], 5), 600, "mixed", 13), (sph(2, [16], 5), 41000, "mixed", 11)):
+        with J.NNAP(model, precision=precision) as p:
+            p.setAutotune(True)
+            log()
+            p.calForces(atoms(n))
+            calls = len(launches("k_neighbors"))
+            assert calls == 3 * shapes + 2, (n, precision, calls)
+            log()
+            p.calForces(atoms(n))
+            assert len(launches("k_neighbors")) == 1
+    """)
